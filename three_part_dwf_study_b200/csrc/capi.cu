@@ -8,6 +8,7 @@
 #include "context.cuh"
 #include "learned.cuh"
 #include "kernels.cuh"
+#include "single.cuh"
 
 using namespace dwfb;
 
@@ -103,8 +104,8 @@ int ensure_workspace(dwf_ctx* c, int nrhs)
     CK(cudaStreamSynchronize(c->stream));
     const size_t f = size_t(nrhs) * c->fsz();
     int st;
-    if ((st = grow(c, c->w_r, f)) || (st = grow(c, c->w_p, f)) || (st = grow(c, c->w_p2, f)) ||
-        (st = grow(c, c->w_t, f)) || (st = grow(c, c->w_p32b, f)) ||
+    if ((st = grow(c, c->w_r, f)) || (st = grow(c, c->w_p, f)) || (st = grow(c, c->w_t, f)) ||
+        (st = grow(c, c->w_p2, size_t(c->fsz()))) || (st = grow(c, c->w_p32b, size_t(c->fsz()))) ||
         (st = grow(c, c->w_b, f)) || (st = grow(c, c->w_x, f)) || (st = grow(c, c->w_r32, f)) ||
         (st = grow(c, c->w_p32, f)) || (st = grow(c, c->w_t32, f)) ||
         (st = grow(c, c->w_e32, f)) || (st = grow(c, c->w_src, f)) ||
@@ -552,32 +553,39 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
     d.bar = c->bar;
     d.timeout_ns = c->timeout_ns;
 
-    // single right-hand side: fused two-barrier iteration; batches: three barriers
-    const bool single = nrhs == 1;
-    const void* fn = mixed ? (single ? reinterpret_cast<const void*>(&cg_mixed_kernel<true, 2>)
-                                     : reinterpret_cast<const void*>(&cg_mixed_kernel<false, 3>))
-                           : (single ? reinterpret_cast<const void*>(&cg64_kernel<true, 2>)
-                                     : reinterpret_cast<const void*>(&cg64_kernel<false, 3>));
-    const size_t smem = solver_smem_bytes(nrhs);
-    CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
-    int bps = 0;
-    CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kSolverThreads, smem));
-    if (bps < 1)
-        return ctx_fail(c, DWF_CUDA_ERROR, "solver kernel cannot be resident");
-    const int cap = bps * c->nsm;
-    int grid_blocks = 0;
-    choose_units(c->L.nsite, nrhs, cap, &d.nch, &d.ch, &grid_blocks);
-    const long units = long(nrhs) * d.nch;
-    int st = ensure_part(c, size_t(units) * 2);
-    if (st)
-        return st;
-    d.part = c->w_part;
-    const int grid = grid_blocks;
-    d.expected_blocks = unsigned(grid);
-    CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
-    void* args[] = {&d};
-    CK(cudaEventRecord(c->ev0, c->stream));
-    CK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolverThreads), args, smem, c->stream));
+    // one right-hand side: the whole-GPU latency kernel; batches: work units
+    int st = DWF_OK;
+    if (nrhs == 1)
+    {
+        if ((st = ensure_part(c, single_part_doubles(c->nsm))))
+            return st;
+        d.part = c->w_part;
+        CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
+        CK(cudaEventRecord(c->ev0, c->stream));
+        CK(launch_single(d, mixed, c->nsm, c->stream));
+    }
+    else
+    {
+        const void* fn = mixed ? reinterpret_cast<const void*>(&cg_mixed_kernel<3>)
+                               : reinterpret_cast<const void*>(&cg64_kernel<3>);
+        const size_t smem = solver_smem_bytes(nrhs);
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+        int bps = 0;
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, kSolverThreads, smem));
+        if (bps < 1)
+            return ctx_fail(c, DWF_CUDA_ERROR, "solver kernel cannot be resident");
+        const int cap = bps * c->nsm;
+        int grid = 0;
+        choose_units(c->L.nsite, nrhs, cap, &d.nch, &d.ch, &grid);
+        if ((st = ensure_part(c, size_t(nrhs) * d.nch * 2)))
+            return st;
+        d.part = c->w_part;
+        d.expected_blocks = unsigned(grid);
+        CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
+        void* args[] = {&d};
+        CK(cudaEventRecord(c->ev0, c->stream));
+        CK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolverThreads), args, smem, c->stream));
+    }
     CK(cudaEventRecord(c->ev1, c->stream));
     c->launches += 1;
     GridBar hb{};

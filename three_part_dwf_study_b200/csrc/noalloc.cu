@@ -21,6 +21,7 @@
 
 #include "context.cuh"
 #include "kernels.cuh"
+#include "single.cuh"
 
 namespace {
 
@@ -165,22 +166,11 @@ extern "C" int dwf_cg_noalloc(const dwf_params* p, int op, const double* theta_d
     d.bar = bar;
     d.timeout_ns = 5000000000ull;
 
-    const void* fn = reinterpret_cast<const void*>(&cg64_kernel<true, 2>);
-    const size_t smem = solver_smem_bytes(1);
-    int bps = 0;
-    if (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) !=
-            cudaSuccess ||
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&bps, fn, 256, smem) != cudaSuccess ||
-        bps < 1)
+    // the kernel and work split of the context-based solver (identical reduction order)
+    if (single_part_doubles(nsm) > size_t(kPartDoubles))
         return DWF_CUDA_ERROR;
-    const long cap = long(bps) * nsm;
-    // the same work units as the context-based solver (identical reduction order)
-    int grid = 0;
-    choose_units(int(nsite), 1, std::min<long>(cap, kMaxUnits), &d.nch, &d.ch, &grid);
     d.part = part;
-    d.expected_blocks = unsigned(grid);
-    void* args[] = {&d};
-    if (cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(256), args, smem, stream) != cudaSuccess)
+    if (launch_single(d, false, nsm, stream) != cudaSuccess)
         return DWF_CUDA_ERROR;
 
     // FP64 true residual |b - A x| / |b| with the scratch temporary t

@@ -11,12 +11,10 @@
 //
 // Reference algorithm (DWF_SOLVER_CG64): domain_wall/include/cg_solver.hpp:17-64.
 // Per iteration, with A = D2 D1 (D1 = D for D^dag D, D^dag for D D^dag):
-//   phase 1: p = r + beta p_old (formed on the fly at every stencil point and
-//            stored at the centre into the other direction buffer),
-//            t = D1 p, |t|^2 = <p, A p>                     | grid barrier
+//   phase 1: t = D1 p, |t|^2 = <p, A p>                     | grid barrier
 //   phase 2: x += alpha p, r -= alpha D2 t, |r|^2           | grid barrier
-// The direction is double-buffered so that phase 1 reads p_old and r at the
-// neighbours while it writes the new p, with no third barrier.
+//   phase 3: p = r + beta p                                 | grid barrier
+// One right-hand side runs in cg_single_kernel (single.cu) instead.
 #include "persist.cuh"
 
 
@@ -25,7 +23,7 @@ using namespace persist;
 namespace {
 }  // namespace
 
-template <bool FUSED, int MINB>
+template <int MINB>
 __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
 {
     const Smem s = carve(d.nrhs);
@@ -54,20 +52,9 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
 
     for (int it = 1; it <= d.maxiter && nact > 0; ++it)
     {
-        double2* pc = (FUSED && !(it & 1)) ? d.p2 : d.p;  // direction of this iteration
-        const double2* po = (pc == d.p) ? d.p2 : d.p;     // previous direction
-        const bool fuse = FUSED && it > 1;
-        // phase 1: p = r + beta p_old, t = D1 p, <p, A p> = |t|^2
+        // phase 1: t = D1 p, <p, A p> = |t|^2
         sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
-            Spinor<double> v;
-            if (!fuse)
-                v = op_site<double>(d, dag1, pc + j * fs, d.U64 + uo, i);
-            else
-            {
-                const DirLd<double> ld{d.r + j * fs, po + j * fs, s.cf[j]};
-                v = op_site_ld<double>(d, dag1, ld, d.U64 + uo, i);
-                st_spinor(pc + j * fs, i, ld.sp(i));
-            }
+            const Spinor<double> v = op_site<double>(d, dag1, d.p + j * fs, d.U64 + uo, i);
             st_spinor(d.t + j * fs, i, v);
             return make_double2(spinor_norm2(v), 0.0);
         });
@@ -92,7 +79,7 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
         sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
             const double a = s.al[j];
             const Spinor<double> ap = op_site<double>(d, !dag1, d.t + j * fs, d.U64 + uo, i);
-            const Spinor<double> p = ld_spinor(pc + j * fs, i);
+            const Spinor<double> p = ld_spinor(d.p + j * fs, i);
             const Spinor<double> x = ld_spinor(d.x + j * fs, i);
             const Spinor<double> r = ld_spinor(d.r + j * fs, i);
             st_spinor(d.x + j * fs, i, axpy(a, p, x));
@@ -122,8 +109,6 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
         }
         __syncthreads();
         nact = compact(d.nrhs, s.act, s.scratch, [&](int j) { return s.state[j] == RHS_ACTIVE; });
-        if (FUSED)
-            continue;
         if (nact == 0)
             break;
         // phase 3: p = r + beta p
@@ -144,7 +129,7 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
 // replaces the residual by the FP64 true residual b - A x whenever the FP32
 // residual has dropped by `delta` since the last update, or when it claims
 // convergence. A right-hand side converges only on the FP64 true residual.
-template <bool FUSED, int MINB>
+template <int MINB>
 __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
 {
     const Smem s = carve(d.nrhs);
@@ -175,19 +160,8 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
     // stall counters live in the upper bits of flag: flag = 2*stalls + update bit
     for (int it = 1; it <= d.maxiter && nact > 0; ++it)
     {
-        float2* pc = (FUSED && !(it & 1)) ? d.p32b : d.p32;
-        const float2* po = (pc == d.p32) ? d.p32b : d.p32;
-        const bool fuse = FUSED && it > 1;
         sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
-            Spinor<float> v;
-            if (!fuse)
-                v = op_site<float>(d, dag1, pc + j * fs, d.U32 + uo, i);
-            else
-            {
-                const DirLd<float> ld{d.r32 + j * fs, po + j * fs, float(s.cf[j])};
-                v = op_site_ld<float>(d, dag1, ld, d.U32 + uo, i);
-                st_spinor(pc + j * fs, i, ld.sp(i));
-            }
+            const Spinor<float> v = op_site<float>(d, dag1, d.p32 + j * fs, d.U32 + uo, i);
             st_spinor(d.t32 + j * fs, i, v);
             return make_double2(spinor_norm2(v), 0.0);
         });
@@ -211,7 +185,7 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
         sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
             const float a = float(s.al[j]);
             const Spinor<float> ap = op_site<float>(d, !dag1, d.t32 + j * fs, d.U32 + uo, i);
-            const Spinor<float> p = ld_spinor(pc + j * fs, i);
+            const Spinor<float> p = ld_spinor(d.p32 + j * fs, i);
             const Spinor<float> e = ld_spinor(d.e32 + j * fs, i);
             const Spinor<float> r = ld_spinor(d.r32 + j * fs, i);
             st_spinor(d.e32 + j * fs, i, axpy(a, p, e));
@@ -290,8 +264,6 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
             __syncthreads();
         }
         nact = compact(d.nrhs, s.act, s.scratch, [&](int j) { return s.state[j] == RHS_ACTIVE; });
-        if (FUSED)
-            continue;
         if (nact == 0)
             break;
         sweep(d, s.act, nact, s.scratch, false, [&](int j, int i, long uo) {
@@ -306,12 +278,9 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
     write_outputs(d, s);
 }
 
-// Instances: the fused two-barrier form at two blocks per SM wins when a
-// single right-hand side is latency bound; the three-barrier form at three
-// blocks per SM wins for batches (fewer loads per site).
-template __global__ void cg64_kernel<true, 2>(SolveDesc);
-template __global__ void cg64_kernel<false, 3>(SolveDesc);
-template __global__ void cg_mixed_kernel<true, 2>(SolveDesc);
-template __global__ void cg_mixed_kernel<false, 3>(SolveDesc);
+// Three blocks per SM: fewer loads in flight per thread, more threads (measured
+// on a 28-right-hand-side batch against two blocks per SM).
+template __global__ void cg64_kernel<3>(SolveDesc);
+template __global__ void cg_mixed_kernel<3>(SolveDesc);
 
 }  // namespace dwfb

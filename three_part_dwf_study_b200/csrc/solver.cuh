@@ -68,9 +68,9 @@ __host__ __device__ inline size_t solver_smem_bytes(int nrhs)
     return 64 * sizeof(double) + size_t(nrhs) * (6 * sizeof(double) + 5 * sizeof(int));
 }
 
-template <bool FUSED, int MINB>
+template <int MINB>
 __global__ void cg64_kernel(SolveDesc d);
-template <bool FUSED, int MINB>
+template <int MINB>
 __global__ void cg_mixed_kernel(SolveDesc d);
 
 }  // namespace dwfb
