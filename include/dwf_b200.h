@@ -385,9 +385,10 @@ int dwf_set_dslash_chunk(dwf_ctx* ctx, int rows);
 
 /* Kernel of the even-odd Schur solve: -1 automatic (default): one thread-
  * block cluster per right-hand side with its FP32 fields in the cluster's
- * distributed shared memory wherever one right-hand side fits (Nt divisible by
- * the cluster size 8 or 16, Ls/4 in {4, 6}, ~200 KB of fields per CTA) and
- * the device can co-schedule such clusters, else the grid-wide persistent
+ * registers and shared memory wherever one right-hand side fits (even Nt and Nx,
+ * Ls <= 24, at most 192 sites of one parity and 227 KB of fields per CTA with 16
+ * CTAs: up to 64x96x16) and the device can co-schedule such clusters, else the
+ * grid-wide persistent
  * kernel; 0 the grid-wide kernel always. The environment variable
  * DWF_B200_EO_KERNEL=grid makes 0 the default of every context. */
 int dwf_set_eo_kernel(dwf_ctx* ctx, int kernel);

@@ -766,7 +766,7 @@ int propagators(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, dou
         // full-lattice solve on D^dag D from it: the reference's
         // stopping rule |D^dag D x - D^dag src| <= rtol |D^dag src| decides.
         std::vector<int> eo_it, eo_ru;
-        const bool clustered = eo_cluster_wave(c) > 0;
+        const bool clustered = eo_cluster_wave(c, nrhs) > 0;
         const double schur_tol = (clustered ? DWFB_EO_SCHUR_TOL : DWFB_EO_SCHUR_TOL_GRID) * rtol;
         st = propagators_eo(c, nrhs, conf_h, src, x, schur_tol, maxiter, eo_it, eo_ru);
         if (st)
@@ -1191,7 +1191,7 @@ int dwf_propagators(dwf_ctx* c, int nrhs, const int* rhs_conf, const double* src
     // the next chunks solve (the copies overlap the solves when the host
     // buffers are page-locked). Each right-hand side's Schur solve is the one
     // a single batch would run; the full-lattice check is decided per chunk.
-    const int wave = solver == DWF_SOLVER_EO_MIXED ? eo_cluster_wave(c) : 0;
+    const int wave = solver == DWF_SOLVER_EO_MIXED ? eo_cluster_wave(c, nrhs) : 0;
     if (wave > 0 && nrhs >= 2 * wave)
         return propagators_pipelined(c, nrhs, rhs_conf, src, x, rtol, maxiter, solver, info,
                                      wave * ((nrhs + DWFB_PIPE_CHUNKS * wave - 1) / (DWFB_PIPE_CHUNKS * wave)));

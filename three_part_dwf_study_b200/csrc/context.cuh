@@ -161,9 +161,10 @@ int set_gauge(dwf_ctx* c, int nconf, const double* theta, cudaMemcpyKind kind);
 int propagators_eo(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, double2* x,
                    double tol, int maxiter, std::vector<int>& iters, std::vector<int>& ru);
 bool eo_eligible(const dwf_ctx* c);
-// Right-hand sides the even-odd cluster solver runs at once on this context's
-// lattice and device (its resident clusters), 0 where the cluster path does not apply.
-int eo_cluster_wave(dwf_ctx* c);
+// Right-hand sides of a batch of nrhs that the even-odd cluster solver runs at
+// once on this context's lattice and device (its resident clusters), 0 where the
+// cluster path does not apply.
+int eo_cluster_wave(dwf_ctx* c, int nrhs);
 // Propagator batch: x = (D^dag D)^-1 D^dag src on device fields.
 int propagators(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, double2* x,
                 double rtol, int maxiter, int solver, dwf_solve_info* info);

@@ -52,12 +52,12 @@ bool eo_eligible(const dwf_ctx* c)
     return c->kind == 0 && c->L.Nt % 2 == 0 && c->L.Nx % 2 == 0 && c->L.diag >= 1.0;
 }
 
-int eo_cluster_wave(dwf_ctx* c)
+int eo_cluster_wave(dwf_ctx* c, int nrhs)
 {
     if (!eo_eligible(c) || c->eo_kernel == 0 || !eo_cluster_enabled())
         return 0;
     EoDesc e{};
-    e.d.nrhs = 1;
+    e.d.nrhs = std::min(nrhs, 2048);
     e.d.delta = 0.1;
     bool ok = false;
     int wave = 0;
@@ -256,6 +256,7 @@ int propagators_eo(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, 
                 int s2 = prepare();
                 if (s2)
                     return s2;
+                CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
                 // external records: event nodes of the graph, not capture markers
                 CK(cudaEventRecordWithFlags(c->ev0, c->stream, cudaEventRecordExternal));
                 bool l = false;
@@ -269,9 +270,13 @@ int propagators_eo(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, 
             if (st)
                 return st;
             std::vector<int> it(n), r(n);
+            GridBar hb{};
             CK(cudaMemcpyAsync(it.data(), c->w_iters, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
             CK(cudaMemcpyAsync(r.data(), c->w_ru, n * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
+            CK(cudaMemcpyAsync(&hb, c->bar, sizeof(GridBar), cudaMemcpyDeviceToHost, c->stream));
             CK(cudaStreamSynchronize(c->stream));
+            if (hb.err != 0)
+                return ctx_fail(c, hb.err, "even-odd cluster solver: a wait ran out");
             float ms = 0.f;
             CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
             c->solver_ms[1] += ms;

@@ -1,80 +1,87 @@
 // Even-odd Schur mixed CG with one thread-block cluster per right-hand side
-// and the FP32 Krylov fields resident in the cluster's shared memory.
+// and the FP32 Krylov fields resident in the cluster's registers and shared
+// memory.
 //
 // The grid-wide kernel (cg_eo_mixed_kernel) runs every right-hand side of a
 // batch in lock step: five grid barriers per iteration across all blocks, the
-// FP32 fields (p, r, e, t, y: ~15 MB per right-hand side-batch each) streaming
-// through L2. Here a cluster of CS CTAs (one per SM) owns one right-hand side
-// at a time: CTA c holds time rows [c R, (c+1) R) (R = Nt / CS) of every field
-// for every fifth-dimension slice in its own shared memory, the stencil reads
-// the rows t0 - 1 and t0 + R of its neighbours through distributed shared
-// memory, and the phases are separated by cluster barriers only. Right-hand
-// sides are independent, so clusters never wait for one another; each takes
-// the right-hand sides cluster_id, cluster_id + nclusters, ...
+// FP32 fields streaming through L2. Here a cluster of CS CTAs owns one
+// right-hand side at a time; CTA c holds time rows [c R, (c+1) R) (R = ceil(Nt /
+// CS), the last CTA may hold fewer) of every field for every fifth-dimension
+// slice, and the phases are separated by cluster barriers only. Right-hand sides
+// are independent, so clusters never wait for one another; each takes the
+// right-hand sides cluster_id, cluster_id + nclusters, ...
 //
-// Per iteration (FP32; the same algebra as cg_eo_mixed_kernel):
-//   P1 (4-D even sites)  y = M5^-1 H_eo p        four lanes per 4-D site
-//   P2 (5-D odd sites)   t = M5 p - H_oe y, |t|^2              | cluster barrier
-//   P3 (4-D even sites)  y = M5^dag^-1 H^dag_eo t               | cluster barrier
-//   P4 (5-D odd sites)   Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap, |r|^2
-//   P5 (5-D odd sites)   p = r + beta p                         | cluster barrier
+// Per iteration (FP32; the same algebra as cg_eo_mixed_kernel), each phase ended
+// by a cluster barrier:
+//   P1 (even sites)  y = M5^-1 H_eo p
+//   P2 (odd sites)   t = M5 p - H_oe y, |t|^2
+//   P3 (even sites)  y = M5^dag^-1 H^dag_eo t
+//   P4 (odd sites)   Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap, |r|^2
+//   P5 (odd sites)   p = r + beta p
+// Shared-memory bandwidth, issue and the latency of the exchanges bound it, so
+//   - only what a neighbour reads is stored in shared memory: NL = 2 or 4 threads
+//     own one 4-D site of each parity, LT = ceil(Ls / NL) slices each, and keep p, r
+//     and (EREG) e of the odd site in registers; M5's fifth-dimension neighbours
+//     come from the thread's own registers and two shuffles. Shared memory holds
+//     two fields, each with one halo row either side: A carries p (read in P1)
+//     and, from P2 on, t (read in P3 and, by its owner, in P4); B carries y;
+//   - lane D q + i of a warp (D = 32 / NL) holds part q of site D w + i, so every
+//     quarter warp reads 128 consecutive bytes;
+//   - halo rows and sums go by asynchronous remote stores counted on mbarriers
+//     (cluster.cuh), so a phase waits for its own CTA (block barrier), in the edge
+//     rows for the neighbouring rows, and for the sums just before their use.
+// A sender may overwrite a halo row once the thread that read it has sent its own
+// row of the same or a later phase back, which every phase waits for: the threads
+// of the first and last row of a CTA send to, and wait for, the same neighbour.
+//
+// 64x64x16, 28 right-hand sides, 443 iterations each (seven clusters of 16, one B200):
+// 28.4 ms with five fields in shared memory, a lane order whose 16-byte reads met
+// on the same banks four ways, a cluster barrier per phase and remote gathers for
+// the sums; 20.6 with p, r, e in registers; 17.6 with asynchronous stores instead of
+// cluster barriers; 16.2 with sums per CTA and no timer read in the waits (a read of
+// the global timer takes about a message's time); 15.4 with fewer reliable updates.
+// 64x96x16 with 56, which the grid-wide kernel had to take: 113 ms, now 45.
+//
+// M5^-1 (per spin an Ls x Ls bidiagonal matrix with the m_f corner, closed form
+// in eo.cuh): the two fifth-dimension recurrences run over the thread's slices in
+// place, the threads' carries are a suffix and a prefix sum with geometric weights
+// c^-k (c = 3 - M5 >= 1) over the site's threads by shuffles, and one multiply-add
+// per slice adds carry and corner term. Ls that does not fill its threads (PAD)
+// leaves slices at the end of the last ones zero.
+//
 // Reliable updates (FP64, fields x, b, t64, y64 in global memory) recompute the
 // residual of the Schur normal equation from x + e when the FP32 residual has
 // fallen by delta^2 since the last one, or convergence is in sight.
-//
-// M5^-1 (per spin an Ls x Ls bidiagonal matrix with the m_f corner, closed
-// form in eo.cuh) is applied by four lanes per 4-D site, each holding Ls/4
-// consecutive slices: the two fifth-dimension recurrences become a suffix and
-// a prefix sum with geometric weights c^-k (c = 3 - M5 >= 1), scanned across
-// the four lanes with shuffles.
-#include <cooperative_groups.h>
-
 #include <algorithm>
 #include <map>
 #include <mutex>
+#include <tuple>
 #include <vector>
 
+#include "cluster.cuh"
 #include "context.cuh"
 #include "eo.cuh"
 #include "persist.cuh"
-
-namespace cg = cooperative_groups;
 
 namespace dwfb {
 
 namespace {
 
-constexpr int kClThreads = 512;
-constexpr int kClMaxLs = 32;
+namespace cg = cooperative_groups;
 
-// Cluster layout: CTA `rank` holds rows t in [rank R, rank R + R) of each
-// parity field; element (s, t, k) (k = x / 2) at local (s R + t - rank R) Nxh + k.
-struct ClGeo
-{
-    int Nt, Nx, Nxh, Vh, Ls, R, CS;
-    int n4;  // 4-D sites of one parity per CTA: R Nxh
-    int n5;  // 5-D sites of one parity per CTA: Ls R Nxh
-};
-
-// Compile-time part of the geometry: rows per CTA, x sites per parity row,
-// slices per lane (Ls = 4 L4). The kernel is instantiated for the shapes the
-// study uses (launch_eo_cluster lists them); integer index arithmetic on them
-// folds to shifts and constants.
-template <int R_, int NXH_, int L4_>
-struct ClShape
-{
-    static constexpr int R = R_, Nxh = NXH_, L4 = L4_, Ls = 4 * L4_;
-    static constexpr int n4 = R * Nxh;   // 4-D sites of one parity per CTA
-    static constexpr int n5 = Ls * n4;   // 5-D sites of one parity per CTA
-    static constexpr int Nx = 2 * Nxh;
-};
+constexpr size_t kClHead = (cl::sum_bytes(3) + 7 * 8 + 15) / 16 * 16;  // sum tables and mbarriers
 
 struct ClDesc
 {
-    ClGeo G;
-    float pw32[kClMaxLs + 1];   // c^-k, k = 0 .. Ls
-    double pw64[kClMaxLs + 1];
-    double delta;               // reliable-update trigger
+    int CS, R;     // CTAs per cluster, time rows per CTA
+    int Nt, Nx, Nxh, Vh, Ls;
+    int SS;        // float4 per slice of a shared field: (R + 2) Nxh
+    float pw32[13];            // c^-k, k = 0 .. 12 (within a thread's slices)
+    float q32[4];              // m_f / (1 + m_f c^-Ls) c^-(LT q): corner weight of the down form per part
+    float u32[4];              // the same of the up form: ... c^-(Ls - LT q - LT)
+    float pad32;               // c^(NL LT - Ls)
+    double pw64[13], q64[4], u64[4], pad64;
+    double delta;              // reliable-update trigger
 };
 
 __device__ __forceinline__ Spinor<float> f4s(float4 v)
@@ -86,285 +93,150 @@ __device__ __forceinline__ float4 s2f4(const Spinor<float>& v)
     return make_float4(v.s0.x, v.s0.y, v.s1.x, v.s1.y);
 }
 
-// Loader of a cluster FP32 field at (s, t, k): rows [t0, t0 + R) from this
-// CTA's own part, the two neighbouring rows t0 - 1 and t0 + R (the only other
-// rows a hop reads) from a halo buffer of this CTA, into which the neighbouring
-// CTAs stored those rows while they computed them (halo_push).
-struct ClRows
-{
-    const float4* halo;  // [2][Ls][Nxh]: row t0 - 1, row t0 + R
-    int t0;
-    int tm;              // row t0 - 1, wrapped: halo slot 0; the other outside row is slot 1
-};
-
-template <class S>
-struct ClLd
-{
-    const float4* base;
-    const ClRows* w;
-    __device__ __forceinline__ Spinor<float> sp(int s, int t, int k) const
-    {
-        const int tl = t - w->t0;
-        if (tl >= 0 && tl < S::R)
-            return f4s(base[(s * S::R + tl) * S::Nxh + k]);
-        const int slot = (t == w->tm) ? 0 : 1;
-        return f4s(w->halo[(slot * S::Ls + s) * S::Nxh + k]);
-    }
-};
-
-// Halo exchange by remote stores: the CTA that computes a value of its first
-// row (tl = 0) also stores it into slot 1 of the halo buffer of CTA rank - 1
-// (whose row t0 + R it is), a value of its last row (tl = R - 1) into slot 0
-// of CTA rank + 1's. The stores need no wait of their own: the cluster barrier
-// that ends the phase makes them visible. Two halo buffers alternate so that a
-// phase reads one while its stores fill the other.
-template <class S>
-struct HaloPush
-{
-    float4* prev;  // halo buffer `dst` of CTA rank - 1 (generic address in the cluster)
-    float4* next;  // of CTA rank + 1
-    __device__ __forceinline__ void put(int s, int tl, int k, float4 v) const
-    {
-        if (tl == 0)
-            prev[(S::Ls + s) * S::Nxh + k] = v;   // slot 1
-        if (tl == S::R - 1)
-            next[s * S::Nxh + k] = v;             // slot 0
-    }
-};
-
-template <class S>
-__device__ __forceinline__ HaloPush<S> halo_to(float4* dst, int CS, int rank)
-{
-    cg::cluster_group cl = cg::this_cluster();
-    return {cl.map_shared_rank(dst, (rank + CS - 1) % CS), cl.map_shared_rank(dst, (rank + 1) % CS)};
-}
-
-// Loader of a global FP64 parity field (s Vh + t Nxh + k).
-template <class S>
-struct GlLd
-{
-    const double2* __restrict__ f;
-    int Vh;
-    __device__ __forceinline__ Spinor<double> sp(int s, int t, int k) const
-    {
-        return ld_spinor(f, long(s) * Vh + t * S::Nxh + k);
-    }
-};
-
-// x (global FP64) + e (cluster FP32).
-template <class S>
-struct XeLd
-{
-    const double2* __restrict__ x;
-    ClLd<S> e;
-    int Vh;
-    __device__ __forceinline__ Spinor<double> sp(int s, int t, int k) const
-    {
-        const Spinor<double> a = ld_spinor(x, long(s) * Vh + t * S::Nxh + k);
-        const Spinor<float> b = e.sp(s, t, k);
-        return {mkc(a.s0.x + double(b.s0.x), a.s0.y + double(b.s0.y)),
-                mkc(a.s1.x + double(b.s1.x), a.s1.y + double(b.s1.y))};
-    }
-};
-
-// Hop term H (H^dag when DAG) at (s, t, x) of the other parity's field read
-// through `ld` (eo_hop with the cluster layout's addressing).
-template <bool DAG, typename R, class S, typename LD>
-__device__ __forceinline__ Spinor<R> cl_hop(const LD& ld, const cplx<R>* __restrict__ U, const Lat& L,
-                                            int Nt, int s, int t, int x)
-{
-    constexpr int Nx = S::Nx;
-    const int tp = (t + 1 == Nt) ? 0 : t + 1;
-    const int tm = (t == 0) ? Nt - 1 : t - 1;
-    const int xp = (x + 1 == Nx) ? 0 : x + 1;
-    const int xm = (x == 0) ? Nx - 1 : x - 1;
-    const Spinor<R> vtp = ld.sp(s, tp, x >> 1);
-    const Spinor<R> vtm = ld.sp(s, tm, x >> 1);
-    const Spinor<R> vxp = ld.sp(s, t, xp >> 1);
-    const Spinor<R> vxm = ld.sp(s, t, xm >> 1);
-    const int here = t * Nx + x;
-    const R stp = (t == Nt - 1) ? R(L.bct) : R(1);
-    const R stm = (t == 0) ? R(L.bct) : R(1);
-    const R sxp = (x == Nx - 1) ? R(L.bcx) : R(1);
-    const R sxm = (x == 0) ? R(L.bcx) : R(1);
-    cplx<R> up, lo;
-    hop4<DAG, R>(vtp, vtm, vxp, vxm, U[here], U[tm * Nx + x], U[L.V + here], U[L.V + t * Nx + xm], stp,
-                 stm, sxp, sxm, up, lo);
-    return {R(-0.5) * up, R(-0.5) * lo};
-}
-
-// M5 (M5^dag when DAG) at (s, t, k) of an odd field read through `ld`
-// (eo_m5 with the cluster layout's addressing).
-template <bool DAG, typename R, typename LD>
-__device__ __forceinline__ Spinor<R> cl_m5(const LD& ld, const Lat& L, int Ls, int s, int t, int k)
-{
-    const Spinor<R> c = ld.sp(s, t, k);
-    const R dg = R(L.diag);
-    Spinor<R> o{dg * c.s0, dg * c.s1};
-    const int sup = (s + 1 == Ls) ? 0 : s + 1;
-    const R cup = (s + 1 == Ls) ? R(L.mf) : R(-1);
-    const int sdn = (s == 0) ? Ls - 1 : s - 1;
-    const R cdn = (s == 0) ? R(L.mf) : R(-1);
-    if (!DAG)
-    {
-        o.s1 += cup * ld.sp(sup, t, k).s1;
-        o.s0 += cdn * ld.sp(sdn, t, k).s0;
-    }
-    else
-    {
-        o.s1 += cdn * ld.sp(sdn, t, k).s1;
-        o.s0 += cup * ld.sp(sup, t, k).s0;
-    }
-    return o;
-}
-
 #define DWFB_SHFL_CPLX(T)                                                                        \
-    __device__ __forceinline__ T shfl_c(T v, int src, int width)                               \
+    __device__ __forceinline__ T lane_c(T v, int src)                                          \
     {                                                                                          \
-        return mkc(__shfl_sync(0xffffffffu, v.x, src, width),                                  \
-                   __shfl_sync(0xffffffffu, v.y, src, width));                                 \
-    }                                                                                          \
-    __device__ __forceinline__ T shfl_dn(T v, int d, int width)                                \
-    {                                                                                          \
-        return mkc(__shfl_down_sync(0xffffffffu, v.x, d, width),                               \
-                   __shfl_down_sync(0xffffffffu, v.y, d, width));                              \
-    }                                                                                          \
-    __device__ __forceinline__ T shfl_up(T v, int d, int width)                                \
-    {                                                                                          \
-        return mkc(__shfl_up_sync(0xffffffffu, v.x, d, width),                                 \
-                   __shfl_up_sync(0xffffffffu, v.y, d, width));                                \
+        return mkc(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));    \
     }
 DWFB_SHFL_CPLX(float2)
 DWFB_SHFL_CPLX(double2)
 #undef DWFB_SHFL_CPLX
 
-// y = M5^-1 z (M5^dag^-1 when DAG) for one 4-D site, the Ls slices spread over
-// the four lanes q of a lane group (lane q holds z[j], s = q L4 + j). Up form
-// (spin DAG ? 0 : 1): y(s) = U(s) - m_f y0 c^-(Ls-s), U(s) = sum_{k>=s} z(k)
-// c^-(k-s+1), y0 = U(0) / (1 + m_f c^-Ls). Down form (the other spin):
-// y(s) = D(s) - m_f yL c^-(s+1), D(s) = sum_{k<=s} z(k) c^-(s-k+1),
-// yL = D(Ls-1) / (1 + m_f c^-Ls). All lanes of the warp take part.
-template <bool DAG, typename R, int L4>
-__device__ __forceinline__ void cl_m5inv(Spinor<R> (&z)[L4], int q, const R* pw, int Ls, R mf)
+// The corner and carry weights of one lane's slices (q = the lane's part).
+template <typename R>
+struct M5w
 {
-    using T = cplx<R>;
-    const R ci = pw[1];
-    // this lane's block totals: T_q = sum_j z_up(j) c^-(j+1) (= U restricted to
-    // the block, at its first slice) and T'_q = sum_j z_dn(j) c^-(L4-j)
-    T Tu = mkc(R(0), R(0)), Td = mkc(R(0), R(0));
-#pragma unroll
-    for (int j = L4 - 1; j >= 0; --j)
-        Tu = ci * ((DAG ? z[j].s0 : z[j].s1) + Tu);
-#pragma unroll
-    for (int j = 0; j < L4; ++j)
-        Td = ci * ((DAG ? z[j].s1 : z[j].s0) + Td);
-    const R cL4 = pw[L4];
-    // suffix scan over lanes of the block totals: B_q = sum_{j>=q} c^-(L4 (j-q)) T_j
-    T B = Tu;
-    {
-        T o = shfl_dn(B, 1, 4);
-        B = (q + 1 < 4) ? B + cL4 * o : B;
-        o = shfl_dn(B, 2, 4);
-        B = (q + 2 < 4) ? B + (cL4 * cL4) * o : B;
-    }
-    // prefix scan: E_q = sum_{j<=q} c^-(L4 (q-j)) T'_j
-    T E = Td;
-    {
-        T o = shfl_up(E, 1, 4);
-        E = (q >= 1) ? E + cL4 * o : E;
-        o = shfl_up(E, 2, 4);
-        E = (q >= 2) ? E + (cL4 * cL4) * o : E;
-    }
-    T carry_u = shfl_dn(B, 1, 4);
-    carry_u = (q + 1 < 4) ? carry_u : mkc(R(0), R(0));
-    T carry_d = shfl_up(E, 1, 4);
-    carry_d = (q >= 1) ? carry_d : mkc(R(0), R(0));
-    const int lane0 = (threadIdx.x & 31) & ~3;
-    const T S = shfl_c(B, lane0, 32);       // U(0), from lane 0 of the group
-    const T Sp = shfl_c(E, lane0 + 3, 32);  // D(Ls-1), from lane 3
-    const R den = R(1) / (R(1) + mf * pw[Ls]);
-    const T y0 = den * S, yL = den * Sp;
-    const int a = q * L4;
-    // up form, in place, downwards: U(s) = U_loc(s) + c^-(L4-j) B_{q+1}
-    T u = mkc(R(0), R(0));
-#pragma unroll
-    for (int j = L4 - 1; j >= 0; --j)
-    {
-        u = ci * ((DAG ? z[j].s0 : z[j].s1) + u);
-        const T yv = u + pw[L4 - j] * carry_u - (mf * pw[Ls - a - j]) * y0;
-        if (DAG)
-            z[j].s0 = yv;
-        else
-            z[j].s1 = yv;
-    }
-    // down form, in place, upwards: D(s) = D_loc(s) + c^-(j+1) E_{q-1}
-    T dn = mkc(R(0), R(0));
-#pragma unroll
-    for (int j = 0; j < L4; ++j)
-    {
-        dn = ci * ((DAG ? z[j].s1 : z[j].s0) + dn);
-        const T yv = dn + pw[j + 1] * carry_d - (mf * pw[a + j + 1]) * yL;
-        if (DAG)
-            z[j].s1 = yv;
-        else
-            z[j].s0 = yv;
-    }
-}
-
-// Deterministic sum over the cluster of one value per CTA: every CTA writes
-// its block sum to red[slot] (own shared memory); after the cluster barrier
-// thread r fetches CTA r's entry into gath[r] and every thread sums gath in
-// rank order, so all CTAs hold the same bits.
-__device__ __forceinline__ double cl_gather(double* red, double* gath, int slot, int CS)
-{
-    if (threadIdx.x < CS)
-        gath[threadIdx.x] = *cg::this_cluster().map_shared_rank(red + slot, threadIdx.x);
-    __syncthreads();
-    double v = 0.0;
-    for (int r = 0; r < CS; ++r)
-        v += gath[r];
-    __syncthreads();
-    return v;
-}
-
-// Cluster barrier (release / acquire at cluster scope): shared memory written
-// before it by any CTA of the cluster is visible to all after it.
-__device__ __forceinline__ void cl_sync() { cg::this_cluster().sync(); }
-
-// The same after phases that write global memory (the FP64 reliable-update
-// fields), with a device-scope fence ahead of the barrier.
-__device__ __forceinline__ void cl_sync_global()
-{
-    __threadfence();
-    cg::this_cluster().sync();
-}
-
-}  // namespace
-
-// A thread's 4-D site in one of the FP32 phases, fixed for the whole solve:
-// where its four hop neighbours sit (slice 0) in the other parity's field.
-// The t neighbours are in this CTA's part (slice stride R Nxh) or in a halo
-// buffer (slice stride Nxh); the x neighbours are always in the own part.
-struct ClNbr
-{
-    int tp, tm;          // offsets of the t+1, t-1 neighbours at slice 0
-    bool tp_own, tm_own;
-    int xp, xm;          // own-part offsets of the x+1, x-1 neighbours at slice 0
+    const R* pw;   // c^-k
+    R qd, qu;      // corner weights (ClDesc q*, u* at q)
+    R pad;
 };
 
-template <class S>
-__device__ __forceinline__ ClNbr cl_nbr(int tl, int x)
+// y = M5^-1 z (M5^dag^-1 when DAG) for one 4-D site, z scaled by c^-1 already,
+// its slices spread over NL lanes at distance D = 32 / NL (part q holds z[j], s = q
+// LT + j, zero where s >= Ls). Up form (spin DAG ? 0 : 1): y(s)
+// = U(s) - m_f y0 c^-(Ls-s), U(s) = sum_{k>=s} z(k) c^-(k-s), y0 = U(0) / (1 +
+// m_f c^-Ls). Down form (the other spin): y(s) = D(s) - m_f yL c^-(s+1), D(s) =
+// sum_{k<=s} z(k) c^-(s-k), yL = D(Ls-1) / (1 + m_f c^-Ls). All lanes of the warp
+// take part.
+template <bool DAG, bool PAD, int NL, typename R, int LT>
+__device__ __forceinline__ void cl_m5inv(Spinor<R> (&z)[LT], int q, const M5w<R>& w)
 {
-    ClNbr n;
-    n.tp_own = tl + 1 < S::R;
-    n.tp = n.tp_own ? (tl + 1) * S::Nxh + (x >> 1) : S::Ls * S::Nxh + (x >> 1);
-    n.tm_own = tl >= 1;
-    n.tm = n.tm_own ? (tl - 1) * S::Nxh + (x >> 1) : (x >> 1);
-    const int xp = (x + 1 == S::Nx) ? 0 : x + 1;
-    const int xm = (x == 0) ? S::Nx - 1 : x - 1;
-    n.xp = tl * S::Nxh + (xp >> 1);
-    n.xm = tl * S::Nxh + (xm >> 1);
-    return n;
+    using T = cplx<R>;
+    constexpr int D = 32 / NL;  // lanes between the parts of a site
+    const R ci = w.pw[1];
+#pragma unroll
+    for (int j = LT - 2; j >= 0; --j)
+    {
+        if (DAG)
+            z[j].s0 += ci * z[j + 1].s0;
+        else
+            z[j].s1 += ci * z[j + 1].s1;
+    }
+#pragma unroll
+    for (int j = 1; j < LT; ++j)
+    {
+        if (DAG)
+            z[j].s1 += ci * z[j - 1].s1;
+        else
+            z[j].s0 += ci * z[j - 1].s0;
+    }
+    const int lane = threadIdx.x & 31;
+    const T zero = mkc(R(0), R(0));
+    T B = DAG ? z[0].s0 : z[0].s1;            // U at the part's first slice
+    T E = DAG ? z[LT - 1].s1 : z[LT - 1].s0;  // D at its last
+    R cL = w.pw[LT];
+#pragma unroll
+    for (int step = 1; step < NL; step *= 2)
+    {
+        const T u = lane_c(B, (lane + step * D) & 31), v = lane_c(E, (lane - step * D) & 31);
+        B += cL * (q + step < NL ? u : zero);  // suffix scan
+        E += cL * (q >= step ? v : zero);      // prefix scan
+        cL *= cL;
+    }
+    T cu = lane_c(B, (lane + D) & 31), cd = lane_c(E, (lane - D) & 31);
+    const T S = lane_c(B, lane & (D - 1));              // U(0)
+    T Sp = lane_c(E, (NL - 1) * D + (lane & (D - 1)));  // D(Ls-1), decayed by the padding
+    if (PAD)
+        Sp = w.pad * Sp;
+    cu = (q + 1 < NL ? cu : zero) - w.qu * S;
+    cd = (q > 0 ? cd : zero) - w.qd * Sp;
+#pragma unroll
+    for (int j = 0; j < LT; ++j)
+    {
+        if (DAG)
+        {
+            z[j].s0 += w.pw[LT - j] * cu;
+            z[j].s1 += w.pw[j + 1] * cd;
+        }
+        else
+        {
+            z[j].s1 += w.pw[LT - j] * cu;
+            z[j].s0 += w.pw[j + 1] * cd;
+        }
+    }
+}
+
+// M5 v (M5^dag v when DAG) for one 4-D site spread over its four lanes.
+template <bool DAG, bool PAD, int NL, int LT>
+__device__ __forceinline__ void cl_m5(const Spinor<float> (&v)[LT], Spinor<float> (&o)[LT], int q, int Ls,
+                                      float dg, float mf)
+{
+    constexpr int D = 32 / NL;
+    const int lane = threadIdx.x & 31;
+    // spin component a(s) needs a(s+1), b(s) needs b(s-1)
+    auto a = [](const Spinor<float>& x) { return DAG ? x.s0 : x.s1; };
+    auto b = [](const Spinor<float>& x) { return DAG ? x.s1 : x.s0; };
+    const float2 up = lane_c(a(v[0]), (lane + D) & 31);       // next lane's first (wraps to s = 0)
+    float2 dn = lane_c(b(v[LT - 1]), (lane - D) & 31);        // previous lane's last
+    float2 first = up;
+    if (PAD)
+    {
+        const int ql = (Ls - 1) / LT, jl = Ls - 1 - ql * LT;
+        first = lane_c(a(v[0]), lane & (D - 1));
+        float2 last = b(v[0]);
+#pragma unroll
+        for (int j = 1; j < LT; ++j)
+            if (j == jl)
+                last = b(v[j]);
+        last = lane_c(last, D * ql + (lane & (D - 1)));
+        if (q == 0)
+            dn = last;
+    }
+#pragma unroll
+    for (int j = 0; j < LT; ++j)
+    {
+        const int s = q * LT + j;
+        const bool top = PAD ? s == Ls - 1 : (j == LT - 1 && q == NL - 1);
+        const float2 na = top ? first : (j + 1 < LT ? a(v[j + 1 < LT ? j + 1 : 0]) : up);
+        const float2 nb = j > 0 ? b(v[j > 0 ? j - 1 : 0]) : dn;
+        const float ca = top ? mf : -1.f, cb = (j == 0 && q == 0) ? mf : -1.f;
+        Spinor<float> r{dg * v[j].s0, dg * v[j].s1};
+        if (DAG)
+        {
+            r.s0 += ca * na;
+            r.s1 += cb * nb;
+        }
+        else
+        {
+            r.s1 += ca * na;
+            r.s0 += cb * nb;
+        }
+        o[j] = r;
+    }
+}
+
+// Where the four hop neighbours of a thread's 4-D site sit in a shared field of
+// the other parity (slice 0; every slice is SS further), halo rows included.
+struct ClNbr
+{
+    int tp, tm, xp, xm;
+};
+
+__device__ __forceinline__ ClNbr cl_nbr(int Nx, int Nxh, int tl, int x)
+{
+    const int xp = (x + 1 == Nx) ? 0 : x + 1, xm = (x == 0) ? Nx - 1 : x - 1;
+    return {(tl + 2) * Nxh + (x >> 1), tl * Nxh + (x >> 1), (tl + 1) * Nxh + (xp >> 1),
+            (tl + 1) * Nxh + (xm >> 1)};
 }
 
 // The four link phases of the hops from (t, x), FP32, boundary signs folded in
@@ -374,9 +246,9 @@ struct ClLinks
     float2 t, tm, x, xm;
 };
 
-__device__ __forceinline__ ClLinks cl_links(const float2* __restrict__ U, const Lat& L, int Nt, int Nx,
-                                            int t, int x)
+__device__ __forceinline__ ClLinks cl_links(const float2* __restrict__ U, const Lat& L, int t, int x)
 {
+    const int Nt = L.Nt, Nx = L.Nx;
     const int tm = (t == 0) ? Nt - 1 : t - 1;
     const int xm = (x == 0) ? Nx - 1 : x - 1;
     const float stp = (t == Nt - 1) ? float(L.bct) : 1.f;
@@ -386,478 +258,747 @@ __device__ __forceinline__ ClLinks cl_links(const float2* __restrict__ U, const 
     return {stp * U[t * Nx + x], stm * U[tm * Nx + x], sxp * U[L.V + t * Nx + x], sxm * U[L.V + t * Nx + xm]};
 }
 
-// Hop term at slice s from precomputed neighbours and links (cl_hop for the
-// FP32 phases): own = the other parity field's own part, halo = its halo buffer.
-template <bool DAG, class S>
-__device__ __forceinline__ Spinor<float> cl_hop_pre(const float4* own, const float4* halo, const ClNbr& n,
-                                                    const ClLinks& u, int s)
+// The hop sum of one slice (times -1/2: H) from a shared field at slice offset so.
+template <bool DAG>
+__device__ __forceinline__ Spinor<float> cl_hop(const float4* f, const ClNbr& n, const ClLinks& u, int so)
 {
-    const float4 a = n.tp_own ? own[n.tp + s * S::n4] : halo[n.tp + s * S::Nxh];
-    const float4 b = n.tm_own ? own[n.tm + s * S::n4] : halo[n.tm + s * S::Nxh];
-    const float4 c = own[n.xp + s * S::n4];
-    const float4 d = own[n.xm + s * S::n4];
     float2 up, lo;
-    hop4<DAG, float>(f4s(a), f4s(b), f4s(c), f4s(d), u.t, u.tm, u.x, u.xm, 1.f, 1.f, 1.f, 1.f, up, lo);
-    return {-0.5f * up, -0.5f * lo};
+    hop4<DAG, float>(f4s(f[n.tp + so]), f4s(f[n.tm + so]), f4s(f[n.xp + so]), f4s(f[n.xm + so]), u.t, u.tm,
+                     u.x, u.xm, 1.f, 1.f, 1.f, 1.f, up, lo);
+    return {up, lo};
 }
 
-// M5 (M5^dag when DAG) at slice s of the own 4-D site h of an odd field.
-template <bool DAG, class S>
-__device__ __forceinline__ Spinor<float> cl_m5_pre(const float4* f, const Lat& L, int s, int h)
+// H (H^dag when DAG) times -1/2 at (s, t, x) of the other parity's global FP64 field.
+template <bool DAG>
+__device__ __forceinline__ Spinor<double> cl_hop64(const double2* __restrict__ f, const double2* __restrict__ U,
+                                                   const Lat& L, int Nxh, long sb, int t, int x)
 {
-    const Spinor<float> c = f4s(f[s * S::n4 + h]);
-    const float dg = float(L.diag);
-    Spinor<float> o{dg * c.s0, dg * c.s1};
-    const int sup = (s + 1 == S::Ls) ? 0 : s + 1;
-    const float cup = (s + 1 == S::Ls) ? float(L.mf) : -1.f;
-    const int sdn = (s == 0) ? S::Ls - 1 : s - 1;
-    const float cdn = (s == 0) ? float(L.mf) : -1.f;
+    const int Nt = L.Nt, Nx = L.Nx;
+    const int tp = (t + 1 == Nt) ? 0 : t + 1, tm = (t == 0) ? Nt - 1 : t - 1;
+    const int xp = (x + 1 == Nx) ? 0 : x + 1, xm = (x == 0) ? Nx - 1 : x - 1;
+    double2 up, lo;
+    hop4<DAG, double>(ld_spinor(f, sb + tp * Nxh + (x >> 1)), ld_spinor(f, sb + tm * Nxh + (x >> 1)),
+                      ld_spinor(f, sb + t * Nxh + (xp >> 1)), ld_spinor(f, sb + t * Nxh + (xm >> 1)),
+                      U[t * Nx + x], U[tm * Nx + x], U[L.V + t * Nx + x], U[L.V + t * Nx + xm],
+                      (t == Nt - 1) ? L.bct : 1.0, (t == 0) ? L.bct : 1.0, (x == Nx - 1) ? L.bcx : 1.0,
+                      (x == 0) ? L.bcx : 1.0, up, lo);
+    return {-0.5 * up, -0.5 * lo};
+}
+
+// M5 (M5^dag when DAG) at slice s of the odd 4-D site h of a global FP64 field.
+template <bool DAG>
+__device__ __forceinline__ Spinor<double> cl_m5_64(const double2* __restrict__ f, const Lat& L, int Ls, long Vh,
+                                                   int s, long h)
+{
+    const Spinor<double> c = ld_spinor(f, s * Vh + h);
+    Spinor<double> o{L.diag * c.s0, L.diag * c.s1};
+    const int sup = (s + 1 == Ls) ? 0 : s + 1, sdn = (s == 0) ? Ls - 1 : s - 1;
+    const double cup = (s + 1 == Ls) ? L.mf : -1.0, cdn = (s == 0) ? L.mf : -1.0;
     if (!DAG)
     {
-        o.s1 += cup * f4s(f[sup * S::n4 + h]).s1;
-        o.s0 += cdn * f4s(f[sdn * S::n4 + h]).s0;
+        o.s1 += cup * ld_spinor(f, sup * Vh + h).s1;
+        o.s0 += cdn * ld_spinor(f, sdn * Vh + h).s0;
     }
     else
     {
-        o.s1 += cdn * f4s(f[sdn * S::n4 + h]).s1;
-        o.s0 += cup * f4s(f[sup * S::n4 + h]).s0;
+        o.s1 += cdn * ld_spinor(f, sdn * Vh + h).s1;
+        o.s0 += cup * ld_spinor(f, sup * Vh + h).s0;
     }
     return o;
 }
 
-// Phase timer of cluster 0, rank 0, thread 0 (only when a phase buffer is
-// given; the same slots as the grid-wide kernel's).
-__device__ __forceinline__ void cl_mark(unsigned long long* ph, int k, unsigned long long& t)
+// Phase timer of the cluster's first thread, kept per right-hand side in shared
+// memory; the longest right-hand side's times and counts are reported.
+struct ClClock
 {
-    if (ph && blockIdx.x == 0 && threadIdx.x == 0)
+    unsigned long long* ph;  // null: off
+    unsigned long long* sm;  // [15]: time of the last mark, ns and counts per phase
+    __device__ __forceinline__ void start() const
     {
-        const unsigned long long n = globaltimer_ns();
-        ph[k] += n - t;
-        ph[8 + k] += 1;
-        t = n;
+        if (!ph)
+            return;
+        for (int k = 1; k < 15; ++k)
+            sm[k] = 0;
+        sm[0] = globaltimer_ns();
     }
+    __device__ __forceinline__ void mark(int k) const
+    {
+        if (!ph)
+            return;
+        const unsigned long long now = globaltimer_ns();
+        sm[1 + k] += now - sm[0];
+        sm[8 + k] += 1;
+        sm[0] = now;
+    }
+    __device__ __forceinline__ void report() const
+    {
+        if (!ph)
+            return;
+        for (int k = 0; k < 7; ++k)
+        {
+            atomicMax(ph + k, sm[1 + k]);
+            atomicMax(ph + 8 + k, sm[8 + k]);
+        }
+    }
+};
+
+// A thread's place: part q of 4-D site h of each parity in its CTA's rows.
+struct ClPlace
+{
+    int q, h, tl, k, t, xe, xo;
+    bool on;
+};
+
+template <int NL>
+__device__ __forceinline__ ClPlace cl_place(const ClDesc& c, int rank)
+{
+    ClPlace w;
+    const int t0 = rank * c.R, rows = min(c.R, c.Nt - t0);
+    constexpr int D = 32 / NL;
+    w.q = int(threadIdx.x & 31) / D;
+    w.h = (int(threadIdx.x) >> 5) * D + int(threadIdx.x & (D - 1));
+    w.on = w.h < rows * c.Nxh;
+    w.tl = w.on ? w.h / c.Nxh : 0;
+    w.k = w.on ? w.h - w.tl * c.Nxh : 0;
+    w.t = t0 + w.tl;
+    w.xe = 2 * w.k + (w.t & 1);
+    w.xo = 2 * w.k + ((w.t + 1) & 1);
+    return w;
 }
 
-template <class S>
-__global__ void __launch_bounds__(kClThreads, 1) cg_eo_cluster_kernel(EoDesc e, ClDesc c)
+// Reliable update in FP64 of right-hand side jr: r = b - Dhat^dag Dhat x with x
+// in global memory (complete before the call); r in FP32 to d.r32 at the thread's
+// own places, |r|^2 of them returned. Kept out of line: it runs once in tens of
+// iterations, and its FP64 temporaries must not take the loop's registers.
+template <int LT, int NL, bool PAD>
+__device__ __noinline__ double cl_reliable(const EoDesc& e, const ClDesc& c, int rank, int jr)
 {
-    constexpr int L4 = S::L4;
     const SolveDesc& d = e.d;
-    const ClGeo G = c.G;
+    const Lat& L = d.L;
+    const ClPlace w = cl_place<NL>(c, rank);
+    const int Ls = c.Ls, Nxh = c.Nxh, s0 = w.q * LT;
+    const long Vh = c.Vh, h64 = long(w.t) * Nxh + w.k;
+    const double2* const U64 = d.U64 + long(d.rhs_conf[jr]) * d.usz;
+    const double2* const xj = d.x + jr * d.fsz;
+    double2* const t64 = d.t + jr * d.fsz;
+    double2* const y64 = e.y64 + jr * d.fsz;
+    const M5w<double> w64{c.pw64, c.q64[w.q], c.u64[w.q], c.pad64};
+    const double ci = c.pw64[1];
+    auto act = [&](int j) { return w.on && (!PAD || s0 + j < Ls); };
+    // y64 = M5^-1 H_eo f (M5^dag^-1 H^dag_eo f)
+    auto hopinv = [&](auto DAG, const double2* f) {
+        constexpr bool dag = decltype(DAG)::value;
+        Spinor<double> z[LT];
+#pragma unroll
+        for (int j = 0; j < LT; ++j)
+        {
+            z[j] = {mkc(0.0, 0.0), mkc(0.0, 0.0)};
+            if (act(j))
+            {
+                const Spinor<double> v = cl_hop64<dag>(f, U64, L, Nxh, (s0 + j) * Vh, w.t, w.xe);
+                z[j] = {ci * v.s0, ci * v.s1};
+            }
+        }
+        cl_m5inv<dag, PAD, NL, double, LT>(z, w.q, w64);
+#pragma unroll
+        for (int j = 0; j < LT; ++j)
+            if (act(j))
+                st_spinor(y64, (s0 + j) * Vh + h64, z[j]);
+    };
+    hopinv(std::false_type{}, xj);
+    cl::sync_global();
+#pragma unroll 2
+    for (int j = 0; j < LT; ++j)
+        if (act(j))
+        {
+            const Spinor<double> m = cl_m5_64<false>(xj, L, Ls, Vh, s0 + j, h64);
+            const Spinor<double> hy = cl_hop64<false>(y64, U64, L, Nxh, (s0 + j) * Vh, w.t, w.xo);
+            st_spinor(t64, (s0 + j) * Vh + h64, Spinor<double>{m.s0 - hy.s0, m.s1 - hy.s1});
+        }
+    cl::sync_global();
+    hopinv(std::true_type{}, t64);
+    cl::sync_global();
+    double a0 = 0.0;
+#pragma unroll 2
+    for (int j = 0; j < LT; ++j)
+        if (act(j))
+        {
+            const Spinor<double> m = cl_m5_64<true>(t64, L, Ls, Vh, s0 + j, h64);
+            const Spinor<double> hy = cl_hop64<true>(y64, U64, L, Nxh, (s0 + j) * Vh, w.t, w.xo);
+            const Spinor<double> b = ld_spinor(d.b + jr * d.fsz, (s0 + j) * Vh + h64);
+            const Spinor<double> v{b.s0 - (m.s0 - hy.s0), b.s1 - (m.s1 - hy.s1)};
+            st_spinor(d.r32 + jr * d.fsz, (s0 + j) * Vh + h64, persist::to32(v));
+            a0 += spinor_norm2(v);
+        }
+    return a0;
+}
+
+}  // namespace
+
+// LT slices per thread, NL threads per site, PAD: NL LT > Ls; EREG: e in registers
+// (else in shared memory). Blocks of up to MAXT threads.
+template <int LT, int NL, bool PAD, bool EREG, int MAXT>
+__global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_constant__ EoDesc e,
+                                                                           const __grid_constant__ ClDesc c)
+{
+    const SolveDesc& d = e.d;
     const Lat& L = d.L;
     cg::cluster_group cluster = cg::this_cluster();
     const int rank = int(cluster.block_rank());
-    const int cid = int(blockIdx.x) / G.CS;
-    const int ncl = int(gridDim.x) / G.CS;
+    const int CS = c.CS, Nxh = c.Nxh, SS = c.SS, Ls = c.Ls;
+    const int cid = int(blockIdx.x) / CS, ncl = int(gridDim.x) / CS;
+    const int rows = min(c.R, c.Nt - rank * c.R);
+    const int prev = (rank + CS - 1) % CS, next = (rank + 1) % CS;
+    const int prows = min(c.R, c.Nt - prev * c.R);
+    __shared__ unsigned long long clk_sm[15];
     extern __shared__ __align__(16) unsigned char cl_smem[];
-    float4* Pf = reinterpret_cast<float4*>(cl_smem);
-    float4* Rf = Pf + S::n5;
-    float4* Ef = Rf + S::n5;
-    float4* Tf = Ef + S::n5;
-    float4* Yf = Tf + S::n5;
-    float4* HA = Yf + S::n5;                     // halo buffers [2][Ls][Nxh] (rows t0 - 1, t0 + R)
-    float4* HB = HA + 2 * S::Ls * S::Nxh;
-    double* red = reinterpret_cast<double*>(HB + 2 * S::Ls * S::Nxh);   // [8] per-CTA partials
-    double* scratch = red + 8;                            // [32] block_sum scratch
-    __shared__ double gath[16];
-    __shared__ float pw32[kClMaxLs + 1];
-    __shared__ double pw64[kClMaxLs + 1];
-    for (int k = threadIdx.x; k <= S::Ls; k += blockDim.x)
-    {
-        pw32[k] = c.pw32[k];
-        pw64[k] = c.pw64[k];
-    }
-    __syncthreads();
-    const int t0 = rank * S::R;
-    // halo buffer A carries p (read in P1), t (P3) and e (reliable update);
-    // B carries y (P2, P4)
-    const ClRows rowsA{HA, t0, (t0 + G.Nt - 1) % G.Nt}, rowsB{HB, t0, (t0 + G.Nt - 1) % G.Nt};
-    const ClLd<S> P{Pf, &rowsA}, E{Ef, &rowsA}, Tl{Tf, &rowsA}, Y{Yf, &rowsB};
-    const HaloPush<S> pushA = halo_to<S>(HA, G.CS, rank), pushB = halo_to<S>(HB, G.CS, rank);
-    // thread roles of the FP32 phases, fixed for the solve: in the 4-D phases
-    // lanes 4h .. 4h+3 take even 4-D site h (lane q: slices q L4 .. q L4 + L4 - 1);
-    // in the 5-D phases thread h + g n4 takes odd 4-D site h and the slices
-    // g, g + G4, ... (G4 = threads / n4 slice groups)
-    static_assert(4 * S::n4 <= kClThreads, "one 4-D site per lane group");
-    constexpr int G4 = kClThreads / S::n4;
-    const int eh = threadIdx.x >> 2;
-    const bool e_on = eh < S::n4;
-    const int etl = e_on ? eh / S::Nxh : 0, ek = e_on ? eh - etl * S::Nxh : 0;
-    const int et = t0 + etl, ex = 2 * ek + (et & 1);
-    const ClNbr enb = cl_nbr<S>(etl, ex);
-    const int oh = threadIdx.x % S::n4, og = threadIdx.x / S::n4;
-    const bool o_on = og < G4;
-    const int otl = oh / S::Nxh, ok = oh - otl * S::Nxh;
-    const int ot = t0 + otl, ox = 2 * ok + ((ot + 1) & 1);
-    const ClNbr onb = cl_nbr<S>(otl, ox);
-    const long fh = d.fsz;  // complex entries of one global parity field
-    const int q = threadIdx.x & 3;
-
-    for (int j = cid; j < d.nrhs; j += ncl)
-    {
-        const long uo = long(d.rhs_conf[j]) * d.usz;
-        const float2* U32 = d.U32 + uo;
-        const double2* U64 = d.U64 + uo;
-        const double2* bj = d.b + j * fh;
-        double2* xj = d.x + j * fh;
-        double2* t64 = d.t + j * fh;
-        double2* y64 = e.y64 + j * fh;
-        const ClLinks eu = cl_links(U32, L, G.Nt, S::Nx, et, ex);
-        const ClLinks ou = cl_links(U32, L, G.Nt, S::Nx, ot, ox);
-        // ---- x = 0: r = b, r32 = p32 = r, e32 = 0; |b|^2 ----
-        double a0 = 0.0;
-        for (int l = threadIdx.x; l < S::n5; l += kClThreads)
-        {
-            const int s = l / S::n4, rem = l - s * S::n4, tl = rem / S::Nxh, k = rem - tl * S::Nxh;
-            const Spinor<double> b = ld_spinor(bj, long(s) * G.Vh + (t0 + tl) * S::Nxh + k);
-            const float4 r32 = s2f4(persist::to32(b));
-            Rf[l] = r32;
-            Pf[l] = r32;
-            pushA.put(s, tl, k, r32);
-            Ef[l] = make_float4(0.f, 0.f, 0.f, 0.f);
-            a0 += spinor_norm2(b);
-        }
-        a0 = block_sum(a0, scratch);
+    double* const tab = reinterpret_cast<double*>(cl_smem);
+    const unsigned bars = cl::smem_addr(cl_smem + cl::sum_bytes(3));  // sums, then halos [A, B][from prev, next]
+    const unsigned hbar = bars + 3 * 8;
+    float4* const FA = reinterpret_cast<float4*>(cl_smem + kClHead);
+    float4* const ES = FA + 2 * Ls * SS;                              // !EREG: e, [LT][threads]
+    float2* const LK = reinterpret_cast<float2*>(ES + (EREG ? 0 : LT * int(blockDim.x)));  // links [even, odd][4][sites]
+    const cl::Sum sum{tab, tab + 3 * cl::kMaxCtas, bars, CS, rank};
+    // lane D q + i of warp w (D = 32 / NL): part q of 4-D site D w + i of each parity
+    const ClPlace pl = cl_place<NL>(c, rank);
+    const int q = pl.q, tl = pl.tl, k = pl.k, t = pl.t;
+    const bool on = pl.on;
+    const int hs = pl.h;
+    const ClNbr en = cl_nbr(c.Nx, Nxh, tl, pl.xe), od = cl_nbr(c.Nx, Nxh, tl, pl.xo);
+    const int own = (tl + 1) * Nxh + k;
+    const int s0 = q * LT;
+    // halo rows: a first row is the previous CTA's row after its last, a last
+    // row the next CTA's row before its first
+    const bool first = on && tl == 0, last = on && tl == rows - 1;
+    const unsigned toprev = cl::map(cl::smem_addr(FA + (prows + 1) * Nxh + k), prev);
+    const unsigned tonext = cl::map(cl::smem_addr(FA + k), next);
+    const unsigned barprev = cl::map(hbar + 8, prev), barnext = cl::map(hbar, next);
+    const int fB = Ls * SS;  // field B behind field A
+    auto act = [&](int j) { return on && (!PAD || s0 + j < Ls); };
+    // The slice stride, opaque: the compiler would otherwise hoist every slice's
+    // address of every phase out of the iteration and spill them.
+    auto stride = [&] {
+        int x = SS;
+        asm volatile("" : "+r"(x));
+        return x;
+    };
+    // v[j] into field A (f = 0) or B (f = fB) at the thread's own place, and to the
+    // CTAs that hold it as a halo row
+    auto store = [&](int f, const Spinor<float> (&v)[LT]) {
+        const int ss = stride();
+        if (on)
+#pragma unroll
+            for (int j = 0; j < LT; ++j)
+                if (!PAD || s0 + j < Ls)
+                    FA[f + (s0 + j) * ss + own] = s2f4(v[j]);
+        if (first)
+#pragma unroll
+            for (int j = 0; j < LT; ++j)
+                if (!PAD || s0 + j < Ls)
+                    cl::send(toprev + unsigned(f + (s0 + j) * ss) * 16u, s2f4(v[j]), barprev + (f ? 16u : 0u));
+        if (last)
+#pragma unroll
+            for (int j = 0; j < LT; ++j)
+                if (!PAD || s0 + j < Ls)
+                    cl::send(tonext + unsigned(f + (s0 + j) * ss) * 16u, s2f4(v[j]), barnext + (f ? 16u : 0u));
+    };
+    // Parities of the barriers: bits 0-2 sums, 3 and 4 the halos of A and B.
+    unsigned par = 0;
+    int bad = 0;
+    // Wait for the halo rows this thread reads from field A (f = 0) or B.
+    auto halo = [&](int f) {
+        const unsigned b = hbar + 16u * f, ph = (par >> (3 + f)) & 1u;
         if (threadIdx.x == 0)
-            red[0] = a0;
-        cl_sync();
-        const double bb = cl_gather(red, gath, 0, G.CS);
-        double rr = bb, rru = bb;
-        int iters = 0, ru = 0, stalls = 0;
-        int state = (bb == 0.0 || persist::converged_now(d, rr, bb)) ? DWF_OK : RHS_ACTIVE;
-
-        unsigned long long ph_t = globaltimer_ns();
-        for (int it = 1; it <= d.maxiter && state == RHS_ACTIVE; ++it)
         {
-            // P1: y = M5^-1 H_eo p (four lanes per even 4-D site)
+            cl::bar_expect(b, unsigned(Ls * Nxh) * 16u);
+            cl::bar_expect(b + 8u, unsigned(Ls * Nxh) * 16u);
+        }
+        // one lane per warp polls for its warp's rows
+        const bool lo = __any_sync(0xffffffffu, first) || threadIdx.x == 0;
+        const bool hi = __any_sync(0xffffffffu, last) || threadIdx.x == 0;
+        if ((threadIdx.x & 31) == 0)
+        {
+            if (lo)
+                bad = bad || !cl::bar_wait(b, ph, d.timeout_ns);
+            if (hi)
+                bad = bad || !cl::bar_wait(b + 8u, ph, d.timeout_ns);
+        }
+        __syncwarp();
+        par ^= 8u << f;
+    };
+    auto total = [&](int slot) {
+        double v;
+        bad |= !sum.get(slot, (par >> slot) & 1u, bad ? 0ull : d.timeout_ns, v);
+        par ^= 1u << slot;
+        return v;
+    };
+    if (threadIdx.x == 0)
+    {
+        for (int i = 0; i < 7; ++i)
+            cl::bar_init(bars + 8u * i);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cl::sync();
+    // !EREG has 80 registers a thread: keep the compiler from holding the next
+    // slice's neighbours while this one's are in use (24 warps hide the latency)
+    auto fence = [] {
+        if (!EREG)
+            asm volatile("" ::: "memory");
+    };
+    const int nsite = int(blockDim.x) / NL;
+    auto links = [&](int i) -> ClLinks {  // 0: even site, 1: odd site
+        const float2* const o = LK + i * 4 * nsite + hs;
+        return {o[0], o[nsite], o[2 * nsite], o[3 * nsite]};
+    };
+    auto eslot = [&](int j) -> float4& { return ES[j * int(blockDim.x) + int(threadIdx.x)]; };
+    const M5w<float> w32{c.pw32, c.q32[q], c.u32[q], c.pad32};
+    const float dg = float(L.diag), mf = float(L.mf);
+    const float zs = -0.5f * c.pw32[1];  // hop factor and c^-1 of M5^-1's input
+    const Spinor<float> zero{make_float2(0.f, 0.f), make_float2(0.f, 0.f)};
+    const long fh = d.fsz, Vh = c.Vh;
+    const long h64 = long(t) * Nxh + k;
+    const ClClock clk{threadIdx.x == 0 && rank == 0 ? e.phase_ns : nullptr, clk_sm};
+
+    for (int jr = cid; jr < d.nrhs; jr += ncl)
+    {
+        // the four links of each of the thread's sites: one copy per site, read
+        // back by its lanes in each phase (16 registers otherwise)
+        if (on && q < 2)
+        {
+            const ClLinks u = cl_links(d.U32 + long(d.rhs_conf[jr]) * d.usz, L, t, q == 0 ? pl.xe : pl.xo);
+            float2* const o = LK + q * 4 * nsite + hs;
+            o[0] = u.t;
+            o[nsite] = u.tm;
+            o[2 * nsite] = u.x;
+            o[3 * nsite] = u.xm;
+        }
+        __syncwarp();
+        // ---- x = 0: r = b (FP32 copy in global memory, field A p = 0); |b|^2 ----
+        double a0 = 0.0;
+#pragma unroll 1
+        for (int j = 0; j < LT; ++j)
+            if (act(j))
             {
-                Spinor<float> z[L4];
-#pragma unroll
-                for (int jj = 0; jj < L4; ++jj)
-                    z[jj] = e_on ? cl_hop_pre<false, S>(Pf, HA, enb, eu, q * L4 + jj) : Spinor<float>{};
-                cl_m5inv<false, float, L4>(z, q, pw32, S::Ls, float(L.mf));
-                if (e_on)
-#pragma unroll
-                    for (int jj = 0; jj < L4; ++jj)
-                    {
-                        const float4 v = s2f4(z[jj]);
-                        Yf[(q * L4 + jj) * S::n4 + eh] = v;
-                        pushB.put(q * L4 + jj, etl, ek, v);
-                    }
+                const Spinor<double> b = ld_spinor(d.b + jr * fh, (s0 + j) * Vh + h64);
+                st_spinor(d.r32 + jr * fh, (s0 + j) * Vh + h64, persist::to32(b));
+                FA[(s0 + j) * SS + own] = make_float4(0.f, 0.f, 0.f, 0.f);
+                a0 += spinor_norm2(b);
             }
-            cl_sync();
-            cl_mark(e.phase_ns, 0, ph_t);
-            // P2: t = M5 p - H_oe y, |t|^2
-            a0 = 0.0;
-            if (o_on)
-                for (int sl = og; sl < S::Ls; sl += G4)
-                {
-                    const Spinor<float> m = cl_m5_pre<false, S>(Pf, L, sl, oh);
-                    const Spinor<float> hy = cl_hop_pre<false, S>(Yf, HB, onb, ou, sl);
-                    const Spinor<float> v{m.s0 - hy.s0, m.s1 - hy.s1};
-                    const float4 v4 = s2f4(v);
-                    Tf[sl * S::n4 + oh] = v4;
-                    pushA.put(sl, otl, ok, v4);
-                    a0 += spinor_norm2(v);
-                }
-            a0 = block_sum(a0, scratch);
-            if (threadIdx.x == 0)
-                red[1] = a0;
-            cl_sync();
-            cl_mark(e.phase_ns, 1, ph_t);
-            const double tt = cl_gather(red, gath, 1, G.CS);
-            if (tt == 0.0 || !isfinite(tt))
+        sum.part(2, a0);
+        __syncthreads();
+        if (threadIdx.x < 32)
+            sum.send(2);
+        const double bb = total(2);
+        double rr = bb, rru = bb, cf = 0.0;
+        int it = 0, ru = 0, stalls = 0;
+        int state = (bb == 0.0 || persist::converged_now(d, rr, bb) || d.maxiter < 1) ? DWF_OK : RHS_ACTIVE;
+        if (state == DWF_OK && !(bb == 0.0 || persist::converged_now(d, rr, bb)))
+            state = DWF_NOT_CONVERGED;
+
+        clk.start();
+        // Between two reliable updates: p and r come from memory (p from field
+        // A's own places), e starts at zero.
+        while (state == RHS_ACTIVE)
+        {
+            Spinor<float> p[LT], r[LT], ev[EREG ? LT : 1];
+#pragma unroll
+            for (int j = 0; j < LT; ++j)
             {
-                state = DWF_NOT_CONVERGED;
-                iters = it;
+                p[j] = act(j) ? f4s(FA[(s0 + j) * SS + own]) : zero;
+                r[j] = act(j) ? ld_spinor(d.r32 + jr * fh, (s0 + j) * Vh + h64) : zero;
+                if (!EREG)
+                    eslot(j) = make_float4(0.f, 0.f, 0.f, 0.f);
+                else
+                    ev[EREG ? j : 0] = zero;
+            }
+            bool want = false;
+            do
+            {
+                ++it;
+                // P5 of the iteration before: p = r + beta p
+                const float beta = float(cf);
+#pragma unroll
+                for (int j = 0; j < LT; ++j)
+                    p[j] = persist::axpy(beta, p[j], r[j]);
+                store(0, p);
+                __syncthreads();
+                clk.mark(6);
+                // P1: y = M5^-1 H_eo p
+                halo(0);
+                {
+                    const ClLinks u = links(0);
+                    const int ss = stride();
+                    Spinor<float> z[LT];
+#pragma unroll
+                    for (int j = 0; j < LT; ++j)
+                        z[j] = zero;
+                    if (on)
+#pragma unroll
+                        for (int j = 0; j < LT; ++j)
+                            if (!PAD || s0 + j < Ls)
+                            {
+                                const Spinor<float> v = cl_hop<false>(FA, en, u, (s0 + j) * ss);
+                                z[j] = {zs * v.s0, zs * v.s1};
+                                fence();
+                            }
+                    cl_m5inv<false, PAD, NL, float, LT>(z, q, w32);
+                    store(fB, z);
+                }
+                __syncthreads();
+                clk.mark(0);
+                // P2: t = M5 p - H_oe y, |t|^2
+                halo(1);
+                a0 = 0.0;
+                {
+                    const ClLinks u = links(1);
+                    const int ss = stride();
+                    Spinor<float> m[LT];
+                    cl_m5<false, PAD, NL, LT>(p, m, q, Ls, dg, mf);
+                    if (on)
+#pragma unroll
+                        for (int j = 0; j < LT; ++j)
+                            if (!PAD || s0 + j < Ls)
+                            {
+                                const Spinor<float> v = cl_hop<false>(FA, od, u, fB + (s0 + j) * ss);
+                                m[j] = persist::axpy(0.5f, v, m[j]);
+                                a0 += spinor_norm2(m[j]);
+                                fence();
+                            }
+                    store(0, m);
+                }
+                sum.part(1, a0);
+                __syncthreads();
+                if (threadIdx.x < 32)
+                    sum.send(1);
+                clk.mark(1);
+                // P3: y = M5^dag^-1 H^dag_eo t
+                halo(0);
+                {
+                    const ClLinks u = links(0);
+                    const int ss = stride();
+                    Spinor<float> z[LT];
+#pragma unroll
+                    for (int j = 0; j < LT; ++j)
+                        z[j] = zero;
+                    if (on)
+#pragma unroll
+                        for (int j = 0; j < LT; ++j)
+                            if (!PAD || s0 + j < Ls)
+                            {
+                                const Spinor<float> v = cl_hop<true>(FA, en, u, (s0 + j) * ss);
+                                z[j] = {zs * v.s0, zs * v.s1};
+                                fence();
+                            }
+                    cl_m5inv<true, PAD, NL, float, LT>(z, q, w32);
+                    store(fB, z);
+                }
+                __syncthreads();
+                clk.mark(3);
+                const double tt = total(1);
+                if (tt == 0.0 || !isfinite(tt))
+                {
+                    state = DWF_NOT_CONVERGED;
+                    break;
+                }
+                const float al = float(rr / tt);
+                clk.mark(2);
+                // P4: Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap; |r|^2
+                halo(1);
+                a0 = 0.0;
+                {
+                    const ClLinks u = links(1);
+                    const int ss = stride();
+                    Spinor<float> tv[LT], m[LT];
+#pragma unroll
+                    for (int j = 0; j < LT; ++j)
+                        tv[j] = act(j) ? f4s(FA[(s0 + j) * ss + own]) : zero;
+                    cl_m5<true, PAD, NL, LT>(tv, m, q, Ls, dg, mf);
+                    if (on)
+#pragma unroll
+                        for (int j = 0; j < LT; ++j)
+                            if (!PAD || s0 + j < Ls)
+                            {
+                                const Spinor<float> v = cl_hop<true>(FA, od, u, fB + (s0 + j) * ss);
+                                const Spinor<float> ap = persist::axpy(0.5f, v, m[j]);
+                                if (!EREG)
+                                    eslot(j) = s2f4(persist::axpy(al, p[j], f4s(eslot(j))));
+                                else
+                                    ev[EREG ? j : 0] = persist::axpy(al, p[j], ev[EREG ? j : 0]);
+                                r[j] = persist::axpy(-al, ap, r[j]);
+                                a0 += spinor_norm2(r[j]);
+                                fence();
+                            }
+                }
+                sum.part(0, a0);
+                __syncthreads();
+                if (threadIdx.x < 32)
+                    sum.send(0);
+                clk.mark(4);
+                const double rn = total(0);
+                if (__syncthreads_or(bad))
+                    break;
+                want = rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
+                cf = rn / rr;
+                rr = rn;
+                clk.mark(5);
+            } while (!want);
+            if (__syncthreads_or(bad))
+                break;
+            if (state != RHS_ACTIVE)
+            {
+                halo(1);  // the y rows on their way
                 break;
             }
-            const float al = float(rr / tt);
-            cl_mark(e.phase_ns, 2, ph_t);
-            // P3: y = M5^dag^-1 H^dag_eo t
-            {
-                Spinor<float> z[L4];
+            // ---- reliable update in FP64: x += e, r = b - Dhat^dag Dhat x ----
 #pragma unroll
-                for (int jj = 0; jj < L4; ++jj)
-                    z[jj] = e_on ? cl_hop_pre<true, S>(Tf, HA, enb, eu, q * L4 + jj) : Spinor<float>{};
-                cl_m5inv<true, float, L4>(z, q, pw32, S::Ls, float(L.mf));
-                if (e_on)
-#pragma unroll
-                    for (int jj = 0; jj < L4; ++jj)
-                    {
-                        const float4 v = s2f4(z[jj]);
-                        Yf[(q * L4 + jj) * S::n4 + eh] = v;
-                        pushB.put(q * L4 + jj, etl, ek, v);
-                    }
-            }
-            cl_sync();
-            cl_mark(e.phase_ns, 3, ph_t);
-            // P4: Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap; |r|^2
-            a0 = 0.0;
-            if (o_on)
-                for (int sl = og; sl < S::Ls; sl += G4)
+            for (int j = 0; j < LT; ++j)
+                if (act(j))
                 {
-                    const int l = sl * S::n4 + oh;
-                    const Spinor<float> m = cl_m5_pre<true, S>(Tf, L, sl, oh);
-                    const Spinor<float> hy = cl_hop_pre<true, S>(Yf, HB, onb, ou, sl);
-                    const Spinor<float> ap{m.s0 - hy.s0, m.s1 - hy.s1};
-                    const Spinor<float> p = f4s(Pf[l]);
-                    const float4 en = s2f4(persist::axpy(al, p, f4s(Ef[l])));
-                    Ef[l] = en;
-                    pushA.put(sl, otl, ok, en);
-                    const Spinor<float> rn = persist::axpy(-al, ap, f4s(Rf[l]));
-                    Rf[l] = s2f4(rn);
-                    a0 += spinor_norm2(rn);
-                }
-            a0 = block_sum(a0, scratch);
-            if (threadIdx.x == 0)
-                red[2] = a0;
-            cl_sync();
-            cl_mark(e.phase_ns, 4, ph_t);
-            const double rn = cl_gather(red, gath, 2, G.CS);
-            iters = it;
-            const bool want = rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) ||
-                              it == d.maxiter;
-            double cf = rn / rr;
-            rr = rn;
-            if (want)
-            {
-                // ---- reliable update in FP64: r = b - Dhat^dag Dhat (x + e) ----
-                const XeLd<S> xe{xj, E, G.Vh};
-                // (a) y64 = M5^-1 H_eo (x + e)
-                for (int w = threadIdx.x; w < 4 * S::n4 + ((4 * S::n4) % 32 ? 32 - (4 * S::n4) % 32 : 0);
-                     w += kClThreads)
-                {
-                    const int h = w >> 2;
-                    const bool on = h < S::n4;
-                    const int tl = on ? h / S::Nxh : 0, k = on ? h - tl * S::Nxh : 0;
-                    const int t = t0 + tl, x = 2 * k + (t & 1);
-                    Spinor<double> z[L4];
-#pragma unroll
-                    for (int jj = 0; jj < L4; ++jj)
-                        z[jj] = on ? cl_hop<false, double, S>(xe, U64, L, G.Nt, q * L4 + jj, t, x) : Spinor<double>{};
-                    cl_m5inv<false, double, L4>(z, q, pw64, S::Ls, L.mf);
-                    if (on)
-#pragma unroll
-                        for (int jj = 0; jj < L4; ++jj)
-                            st_spinor(y64, long(q * L4 + jj) * G.Vh + t * S::Nxh + k, z[jj]);
-                }
-                cl_sync_global();
-                // (b) t64 = M5 (x + e) - H_oe y64
-                const GlLd<S> yl{y64, G.Vh};
-                for (int l = threadIdx.x; l < S::n5; l += kClThreads)
-                {
-                    const int s = l / S::n4, rem = l - s * S::n4, tl = rem / S::Nxh, k = rem - tl * S::Nxh;
-                    const int t = t0 + tl, x = 2 * k + ((t + 1) & 1);
-                    const Spinor<double> m = cl_m5<false, double>(xe, L, S::Ls, s, t, k);
-                    const Spinor<double> hy = cl_hop<false, double, S>(yl, U64, L, G.Nt, s, t, x);
-                    st_spinor(t64, long(s) * G.Vh + t * S::Nxh + k, Spinor<double>{m.s0 - hy.s0, m.s1 - hy.s1});
-                }
-                cl_sync_global();
-                // (c) y64 = M5^dag^-1 H^dag_eo t64
-                const GlLd<S> tlg{t64, G.Vh};
-                for (int w = threadIdx.x; w < 4 * S::n4 + ((4 * S::n4) % 32 ? 32 - (4 * S::n4) % 32 : 0);
-                     w += kClThreads)
-                {
-                    const int h = w >> 2;
-                    const bool on = h < S::n4;
-                    const int tl = on ? h / S::Nxh : 0, k = on ? h - tl * S::Nxh : 0;
-                    const int t = t0 + tl, x = 2 * k + (t & 1);
-                    Spinor<double> z[L4];
-#pragma unroll
-                    for (int jj = 0; jj < L4; ++jj)
-                        z[jj] = on ? cl_hop<true, double, S>(tlg, U64, L, G.Nt, q * L4 + jj, t, x) : Spinor<double>{};
-                    cl_m5inv<true, double, L4>(z, q, pw64, S::Ls, L.mf);
-                    if (on)
-#pragma unroll
-                        for (int jj = 0; jj < L4; ++jj)
-                            st_spinor(y64, long(q * L4 + jj) * G.Vh + t * S::Nxh + k, z[jj]);
-                }
-                cl_sync_global();
-                // (d) r = b - (M5^dag t64 - H^dag_oe y64); x += e; r32 = r; e = 0
-                a0 = 0.0;
-                for (int l = threadIdx.x; l < S::n5; l += kClThreads)
-                {
-                    const int s = l / S::n4, rem = l - s * S::n4, tl = rem / S::Nxh, k = rem - tl * S::Nxh;
-                    const int t = t0 + tl, x = 2 * k + ((t + 1) & 1);
-                    const long gi = long(s) * G.Vh + t * S::Nxh + k;
-                    const Spinor<double> m = cl_m5<true, double>(tlg, L, S::Ls, s, t, k);
-                    const Spinor<double> hy = cl_hop<true, double, S>(yl, U64, L, G.Nt, s, t, x);
-                    const Spinor<double> b = ld_spinor(bj, gi);
-                    const Spinor<double> r{b.s0 - (m.s0 - hy.s0), b.s1 - (m.s1 - hy.s1)};
+                    double2* const xj = d.x + jr * fh;
+                    const long gi = (s0 + j) * Vh + h64;
                     const Spinor<double> xo = ld_spinor(xj, gi);
-                    const Spinor<float> ev = f4s(Ef[l]);
-                    st_spinor(xj, gi, Spinor<double>{mkc(xo.s0.x + double(ev.s0.x), xo.s0.y + double(ev.s0.y)),
-                                                     mkc(xo.s1.x + double(ev.s1.x), xo.s1.y + double(ev.s1.y))});
-                    Rf[l] = s2f4(persist::to32(r));
-                    Ef[l] = make_float4(0.f, 0.f, 0.f, 0.f);
-                    a0 += spinor_norm2(r);
+                    const Spinor<double> de = persist::to64(!EREG ? f4s(eslot(j)) : ev[EREG ? j : 0]);
+                    st_spinor(xj, gi, Spinor<double>{xo.s0 + de.s0, xo.s1 + de.s1});
+                    FA[(s0 + j) * SS + own] = s2f4(p[j]);
                 }
-                a0 = block_sum(a0, scratch);
-                if (threadIdx.x == 0)
-                    red[3] = a0;
-                cl_sync_global();
-                const double rt = cl_gather(red, gath, 3, G.CS);
-                ru += 1;
-                cf = cf * (rt / rr);
-                stalls = (rt >= 0.5 * rru) ? stalls + 1 : 0;
-                rr = rt;
-                rru = rt;
-                if (persist::converged_now(d, rt, bb))
-                    state = DWF_OK;
-                else if (!isfinite(rt) || stalls >= d.stall_limit || it == d.maxiter)
-                    state = DWF_NOT_CONVERGED;
-                if (state != RHS_ACTIVE)
-                    break;
-            }
-            cl_mark(e.phase_ns, 5, ph_t);
-            // P5: p = r + beta p
-            const float beta = float(cf);
-            if (o_on)
-                for (int sl = og; sl < S::Ls; sl += G4)
-                {
-                    const int l = sl * S::n4 + oh;
-                    const float4 v = s2f4(persist::axpy(beta, f4s(Pf[l]), f4s(Rf[l])));
-                    Pf[l] = v;
-                    pushA.put(sl, otl, ok, v);
-                }
-            cl_sync();
-            cl_mark(e.phase_ns, 6, ph_t);
+            cl::sync_global();
+            a0 = cl_reliable<LT, NL, PAD>(e, c, rank, jr);
+            sum.part(2, a0);
+            __syncthreads();
+            if (threadIdx.x < 32)
+                sum.send(2);
+            const double rt = total(2);
+            ru += 1;
+            cf = cf * (rt / rr);
+            stalls = (rt >= 0.5 * rru) ? stalls + 1 : 0;
+            rr = rt;
+            rru = rt;
+            if (persist::converged_now(d, rt, bb))
+                state = DWF_OK;
+            else if (!isfinite(rt) || stalls >= d.stall_limit || it == d.maxiter)
+                state = DWF_NOT_CONVERGED;
+            clk.mark(5);
         }
+        if (__syncthreads_or(bad))
+        {
+            if (threadIdx.x == 0)
+                raise_error(d.bar, DWF_TIMEOUT);
+            cl::linger(d.timeout_ns);
+            return;
+        }
+        clk.report();
         if (rank == 0 && threadIdx.x == 0)
         {
-            d.out_iters[j] = iters;
-            d.out_status[j] = state == RHS_ACTIVE ? DWF_NOT_CONVERGED : state;
-            d.out_relres[j] = bb > 0.0 ? sqrt(rr / bb) : 0.0;
-            d.out_ru[j] = ru;
+            d.out_iters[jr] = it;
+            d.out_status[jr] = state;
+            d.out_relres[jr] = bb > 0.0 ? sqrt(rr / bb) : 0.0;
+            d.out_ru[jr] = ru;
         }
         // the next right-hand side overwrites the fields and partials
-        cl_sync();
+        cl::sync();
     }
 }
 
-// shapes: 64x64x16 (16-CTA clusters), 64x32x16 and 32x32x16 (8-CTA),
-// 64x56x16 (16-CTA), 32x16x24 (8-CTA)
-#define DWFB_CL_SHAPES(X) X(4, 32, 4) X(8, 16, 4) X(4, 16, 4) X(4, 28, 4) X(4, 8, 6)
-#define DWFB_CL_INST(r, h, l) template __global__ void cg_eo_cluster_kernel<ClShape<r, h, l>>(EoDesc, ClDesc);
-DWFB_CL_SHAPES(DWFB_CL_INST)
-#undef DWFB_CL_INST
+namespace {
+
+// Kernel forms. Two threads per site hold more slices each (fewer instructions
+// for places, links, sums and waits per slice, more registers a thread); four
+// where Ls needs it. X(form, LT, NL, PAD, EREG, MAXT)
+#define DWFB_CL_PADS(X, lt, nl, er, mt) X(lt, nl, false, er, mt) X(lt, nl, true, er, mt)
+#define DWFB_CL_FORM2(X, er, mt)                                                                  \
+    DWFB_CL_PADS(X, 1, 2, er, mt) DWFB_CL_PADS(X, 2, 2, er, mt) DWFB_CL_PADS(X, 3, 2, er, mt)     \
+    DWFB_CL_PADS(X, 4, 2, er, mt) DWFB_CL_PADS(X, 5, 2, er, mt) DWFB_CL_PADS(X, 6, 2, er, mt)     \
+    DWFB_CL_PADS(X, 7, 2, er, mt) DWFB_CL_PADS(X, 8, 2, er, mt)
+#define DWFB_CL_FORM4(X, er, mt)                                                                  \
+    DWFB_CL_PADS(X, 1, 4, er, mt) DWFB_CL_PADS(X, 2, 4, er, mt) DWFB_CL_PADS(X, 3, 4, er, mt)     \
+    DWFB_CL_PADS(X, 4, 4, er, mt) DWFB_CL_PADS(X, 5, 4, er, mt) DWFB_CL_PADS(X, 6, 4, er, mt)
+#define DWFB_CL_KERNELS(X) \
+    DWFB_CL_FORM2(X, true, 256) DWFB_CL_FORM2(X, false, 384) DWFB_CL_FORM4(X, true, 512) DWFB_CL_FORM4(X, false, 768)
+
+struct ClShape
+{
+    int CS = 0, R = 0, NL = 0, LT = 0, threads = 0, maxt = 0, resident = 0;
+    bool ereg = false;
+    size_t smem = 0;
+    const void* fn = nullptr;
+};
+
+size_t cl_smem_bytes(const Lat& L, const ClShape& s)
+{
+    return kClHead + size_t(2) * L.Ls * (s.R + 2) * (L.Nx / 2) * sizeof(float4) +
+           size_t(8) * (s.threads / s.NL) * sizeof(float2) +
+           (s.ereg ? 0 : size_t(s.LT) * s.threads * sizeof(float4));
+}
+
+constexpr size_t kClSmemMax = 227 * 1024 - 128;  // 128 bytes are static
+
+const void* cl_kernel(const ClShape& s, bool pad)
+{
+#define DWFB_CL_PICK(lt, nl, p, er, mt)                                            \
+    if (s.LT == lt && s.NL == nl && pad == p && s.ereg == er && s.maxt == mt)      \
+        return reinterpret_cast<const void*>(&cg_eo_cluster_kernel<lt, nl, p, er, mt>);
+    DWFB_CL_KERNELS(DWFB_CL_PICK)
+#undef DWFB_CL_PICK
+    return nullptr;
+}
+
+void cl_config(const ClShape& sh, int clusters, cudaStream_t stream, cudaLaunchConfig_t& cfg,
+               cudaLaunchAttribute& attr)
+{
+    attr.id = cudaLaunchAttributeClusterDimension;
+    attr.val.clusterDim.x = unsigned(sh.CS);
+    attr.val.clusterDim.y = 1;
+    attr.val.clusterDim.z = 1;
+    cfg = cudaLaunchConfig_t{};
+    cfg.gridDim = dim3(unsigned(sh.CS * clusters));
+    cfg.blockDim = dim3(unsigned(sh.threads));
+    cfg.dynamicSmemBytes = sh.smem;
+    cfg.stream = stream;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+}
+
+// Clusters of this shape resident at once on the device (kernel attributes set
+// on the way), queried once per device and shape, so that a later call, the one
+// a stream capture records, issues the launch alone. 0: none.
+int cl_resident(const ClShape& sh, int device)
+{
+    using Key = std::tuple<int, const void*, int, int, size_t>;
+    static std::map<Key, int> known;
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lock(mu);
+    const Key key(device, sh.fn, sh.CS, sh.threads, sh.smem);
+    const auto it = known.find(key);
+    if (it != known.end())
+        return it->second;
+    int n = 0;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    cl_config(sh, 1, nullptr, cfg, attr);
+    if (cudaFuncSetAttribute(sh.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kClSmemMax)) != cudaSuccess ||
+        cudaFuncSetAttribute(sh.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
+        cudaOccupancyMaxActiveClusters(&n, sh.fn, &cfg) != cudaSuccess)
+    {
+        cudaGetLastError();
+        n = 0;
+    }
+    known[key] = n;
+    return n;
+}
+
+// Cluster shape for a batch: the rows per CTA for which the estimated time of an
+// iteration over the whole batch is least. An iteration of one cluster takes
+// about 3.5 us of latencies (five phases, two sums) plus 0.09 us per warp and
+// slice of a CTA at four threads per site, 0.08 at two, more where CTAs share an SM; the batch takes
+// as many rounds as its right-hand sides need of the resident clusters, whose
+// number falls with the CTAs per cluster (a cluster sits in one GPC: 7 clusters of
+// 16 fit, 16 of 8). Measured: 64x64x16 with 28 right-hand sides 16.2 ms at 16 CTAs,
+// 26 at 11; 64x32x16 with 112: 30.6 at 8 CTAs, 50 at 16; 48x40x12 with 20: 6.3 at 16
+// CTAs, 6.1 at 8, 3.9 at 6; 64x96x16 with 56: two threads per site 46.4, four 54.7.
+ClShape cl_shape(const dwf_ctx* c, int nrhs)
+{
+    const Lat& L = c->L;
+    ClShape best;
+    const int Nxh = L.Nx / 2;
+    if (L.Ls > 24 || L.Nt % 2 != 0 || L.Nx % 2 != 0)
+        return best;
+    double least = 0.0;
+    for (int R = L.Nt; R >= 1; --R)
+    {
+        const int CS = (L.Nt + R - 1) / R;
+        if (CS > cl::kMaxCtas)
+            break;
+        if (R > 1 && (L.Nt + R - 2) / (R - 1) == CS)
+            continue;  // fewer rows per CTA with as many CTAs
+        for (int form = 0; form < 4; ++form)
+        {
+            ClShape sh;
+            sh.R = R;
+            sh.CS = CS;
+            sh.NL = form < 2 ? 2 : 4;
+            sh.LT = (L.Ls + sh.NL - 1) / sh.NL;
+            sh.ereg = form % 2 == 0;
+            sh.maxt = form == 0 ? 256 : form == 1 ? 384 : form == 2 ? 512 : 768;
+            const int D = 32 / sh.NL;
+            sh.threads = (R * Nxh + D - 1) / D * 32;
+            sh.smem = cl_smem_bytes(L, sh);
+            if (sh.threads > sh.maxt || sh.smem > kClSmemMax)
+                continue;
+            sh.fn = cl_kernel(sh, sh.NL * sh.LT != L.Ls);
+            if (!sh.fn || (sh.resident = cl_resident(sh, c->device)) < 1)
+                continue;
+            const int used = std::min(sh.resident, nrhs);
+            const double share = std::max(1.0, double(used) * sh.CS / c->nsm);
+            const double rounds = (nrhs + used - 1) / used;
+            const double t = rounds * (3.5 + (sh.NL == 4 ? 0.09 : 0.08) * (sh.threads / 32) * sh.LT * share);
+            if (best.CS == 0 || t < least)
+            {
+                best = sh;
+                least = t;
+            }
+            break;
+        }
+    }
+    return best;
+}
+
+}  // namespace
 
 // Launch the cluster solver for a batch prepared by propagators_eo (fields in
 // EoDesc as for cg_eo_mixed_kernel). Returns DWF_BAD_ARG (nothing launched)
 // when the lattice or the device does not allow it: the caller then runs the
-// grid-wide kernel. A dry call only checks, and reports in *wave (when not
+// grid-wide kernel. dry: only check that the cluster kernel takes this batch and
+// prepare its launch; *launched tells whether it would launch, *wave (when not
 // null) how many right-hand sides the resident clusters solve at once.
-// Launch shape of the cluster kernel per (device, kernel): attributes set and
-// the resident-cluster count queried once, so that a later call (the one a
-// stream capture records) issues the launch alone.
-struct ClLaunchShape
-{
-    int nclust = 0;
-};
-
-// dry: check that the cluster kernel takes this batch and prepare its launch
-// shape without launching (*launched tells whether it would launch).
 int launch_eo_cluster(dwf_ctx* c, EoDesc& e, bool* launched, bool dry, int* wave)
 {
-    static std::map<std::pair<int, const void*>, ClLaunchShape> shapes;
-    static std::mutex shapes_mu;
     *launched = false;
     const Lat& L = c->L;
-    const int Ls = L.Ls;
-    if (Ls % 4 != 0 || Ls > kClMaxLs)
+    const ClShape sh = cl_shape(c, std::max(1, e.d.nrhs));
+    if (!sh.fn)
         return DWF_BAD_ARG;
-    ClDesc cd{};
-    ClGeo& G = cd.G;
-    G.Nt = L.Nt;
-    G.Nx = L.Nx;
-    G.Nxh = L.Nx / 2;
-    G.Vh = L.V / 2;
-    G.Ls = Ls;
-    int CS = 0;
-    size_t smem = 0;
-    for (int cs : {8, 16})
-    {
-        if (L.Nt % cs != 0)
-            continue;
-        const int R = L.Nt / cs;
-        const int n5 = Ls * R * G.Nxh;
-        const size_t sm = size_t(5) * n5 * sizeof(float4) + size_t(4) * Ls * G.Nxh * sizeof(float4) +
-                          40 * sizeof(double);
-        // one right-hand side's fields must fit the cluster's shared memory and
-        // the lane groups of the 4-D phases must fill whole warps
-        if (sm <= size_t(200 * 1024) && (R * G.Nxh) % 8 == 0)
-        {
-            CS = cs;
-            smem = sm;
-            G.R = R;
-            G.n4 = R * G.Nxh;
-            G.n5 = n5;
-            break;
-        }
-    }
-    if (CS == 0)
-        return DWF_BAD_ARG;
-    G.CS = CS;
-    const double cc = L.diag;
-    double p = 1.0;
-    for (int k = 0; k <= Ls; ++k)
-    {
-        cd.pw64[k] = p;
-        cd.pw32[k] = float(p);
-        p /= cc;
-    }
-    cd.delta = e.d.delta;
-    const void* fn = nullptr;
-#define DWFB_CL_PICK(r, h, l)                                                              \
-    if (G.R == r && G.Nxh == h && Ls == 4 * l)                                             \
-        fn = reinterpret_cast<const void*>(&cg_eo_cluster_kernel<ClShape<r, h, l>>);
-    DWFB_CL_SHAPES(DWFB_CL_PICK)
-#undef DWFB_CL_PICK
-    if (!fn)
-        return DWF_BAD_ARG;
-    std::lock_guard<std::mutex> lock(shapes_mu);
-    ClLaunchShape& sh = shapes[std::make_pair(c->device, fn)];
-    if (sh.nclust == 0 &&
-        (cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)) != cudaSuccess ||
-         (CS > 8 && cudaFuncSetAttribute(fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess)))
-    {
-        cudaGetLastError();
-        return DWF_BAD_ARG;
-    }
-    cudaLaunchConfig_t cfg{};
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = unsigned(CS);
-    attr[0].val.clusterDim.y = 1;
-    attr[0].val.clusterDim.z = 1;
-    cfg.blockDim = dim3(kClThreads);
-    cfg.dynamicSmemBytes = smem;
-    cfg.stream = c->stream;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    cfg.gridDim = dim3(unsigned(CS * std::max(1, e.d.nrhs)));
-    if (sh.nclust == 0)
-    {
-        int nc = 0;
-        if (cudaOccupancyMaxActiveClusters(&nc, fn, &cfg) != cudaSuccess || nc < 1)
-        {
-            cudaGetLastError();
-            return DWF_BAD_ARG;
-        }
-        sh.nclust = nc;
-    }
     if (dry)
     {
         *launched = true;
         if (wave)
-            *wave = sh.nclust;
+            *wave = sh.resident;
         return DWF_OK;
     }
-    const int nclust = std::min(sh.nclust, e.d.nrhs);
-    cfg.gridDim = dim3(unsigned(CS * nclust));
+    ClDesc cd{};
+    cd.CS = sh.CS;
+    cd.R = sh.R;
+    cd.Nt = L.Nt;
+    cd.Nx = L.Nx;
+    cd.Nxh = L.Nx / 2;
+    cd.Vh = L.V / 2;
+    cd.Ls = L.Ls;
+    cd.SS = (sh.R + 2) * cd.Nxh;
+    const double cc = L.diag;
+    auto pw = [&](int k) {
+        double p = 1.0;
+        for (int i = 0; i < std::abs(k); ++i)
+            p = k > 0 ? p / cc : p * cc;
+        return p;
+    };
+    for (int k = 0; k <= 12; ++k)
+        cd.pw32[k] = float(cd.pw64[k] = pw(k));
+    const double corner = L.mf / (1.0 + L.mf * pw(L.Ls));
+    for (int q = 0; q < sh.NL; ++q)
+    {
+        cd.q32[q] = float(cd.q64[q] = corner * pw(sh.LT * q));
+        cd.u32[q] = float(cd.u64[q] = corner * pw(L.Ls - sh.LT * q - sh.LT));
+    }
+    cd.pad32 = float(cd.pad64 = pw(L.Ls - sh.NL * sh.LT));
+    // Fewer reliable updates than the grid kernel's delta of 0.1 asks for: one costs
+    // about four iterations here. 64x64x16, 28 right-hand sides to 1e-12: 0.1 -> 12
+    // updates, 16.2 ms; 0.03 -> 8, 15.5; 0.01 -> 6, 15.2; 24x20x8 needs 184, 188, 190
+    // iterations there, and 213 at 0.003.
+    cd.delta = 0.02;
+    cudaLaunchConfig_t cfg;
+    cudaLaunchAttribute attr;
+    cl_config(sh, std::min(sh.resident, e.d.nrhs), c->stream, cfg, attr);
     void* args[] = {&e, &cd};
-    if (cudaLaunchKernelExC(&cfg, fn, args) != cudaSuccess)
+    if (cudaLaunchKernelExC(&cfg, sh.fn, args) != cudaSuccess)
         return ctx_fail(c, DWF_CUDA_ERROR, "even-odd cluster solver: launch failed");
     *launched = true;
     return DWF_OK;

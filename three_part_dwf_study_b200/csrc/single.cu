@@ -142,15 +142,17 @@ struct GridSum
     unsigned long long limit_ns;
     unsigned tag;
 
+    // The timer is read only now and then: a read takes about as long as the
+    // message it waits for.
     __device__ __forceinline__ bool poll(const ulonglong2* p, double& u) const
     {
-        if (slot_load(p, tag, u))
-            return true;
+        for (int n = 0; n < 256; ++n)
+            if (slot_load(p, tag, u))
+                return true;
         const unsigned long long t0 = globaltimer_ns();
-        unsigned n = 0;
-        while (!slot_load(p, tag, u))
+        for (unsigned n = 1; !slot_load(p, tag, u); ++n)
         {
-            if ((++n & 63u) != 0)
+            if (n % 64u != 0)
                 continue;
             cuda::atomic_ref<int, cuda::thread_scope_device> err(bar->err);
             if (err.load(cuda::memory_order_relaxed) != 0)
