@@ -5,6 +5,7 @@
 #include <cstring>
 #include <vector>
 
+#include "cg_cluster.cuh"
 #include "context.cuh"
 #include "learned.cuh"
 #include "kernels.cuh"
@@ -553,18 +554,21 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
     d.bar = c->bar;
     d.timeout_ns = c->timeout_ns;
 
-    // one right-hand side: the whole-GPU latency kernel; batches: work units
+    // lattices that fit a cluster: one cluster per right-hand side; else one
+    // right-hand side: the whole-GPU latency kernel, batches: work units
     int st = DWF_OK;
-    if (nrhs == 1)
+    bool clustered = false;
+    CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
+    CK(cudaEventRecord(c->ev0, c->stream));
+    CK(launch_cg_cluster(d, mixed, c->device, c->nsm, c->stream, &clustered));
+    if (!clustered && nrhs == 1)
     {
         if ((st = ensure_part(c, single_part_doubles(c->nsm))))
             return st;
         d.part = c->w_part;
-        CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
-        CK(cudaEventRecord(c->ev0, c->stream));
         CK(launch_single(d, mixed, c->nsm, c->stream));
     }
-    else
+    else if (!clustered)
     {
         const void* fn = mixed ? reinterpret_cast<const void*>(&cg_mixed_kernel<3>)
                                : reinterpret_cast<const void*>(&cg64_kernel<3>);
@@ -581,9 +585,7 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
             return st;
         d.part = c->w_part;
         d.expected_blocks = unsigned(grid);
-        CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
         void* args[] = {&d};
-        CK(cudaEventRecord(c->ev0, c->stream));
         CK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolverThreads), args, smem, c->stream));
     }
     CK(cudaEventRecord(c->ev1, c->stream));
@@ -604,7 +606,7 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
     c->solver_ms[0] += ms;
     c->solver_launches[0] += 1;
     if (hb.err != 0)
-        return ctx_fail(c, hb.err, hb.err == DWF_TIMEOUT ? "persistent solver: a grid barrier wait ran out"
+        return ctx_fail(c, hb.err, hb.err == DWF_TIMEOUT ? "persistent solver: a wait ran out"
                                                           : "persistent solver: device error");
     return DWF_OK;
 }

@@ -1,0 +1,13 @@
+// Full-lattice CG with one thread-block cluster per right-hand side (cg_cluster.cu).
+#pragma once
+
+#include "solver.cuh"
+
+namespace dwfb {
+
+// Solve d's right-hand sides on the cluster kernel if the lattice fits one and the
+// kernel is estimated faster than the grid-wide ones for this batch; *taken tells.
+// d.bar is zeroed; d.part is not used.
+cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cudaStream_t stream, bool* taken);
+
+}  // namespace dwfb

@@ -1,5 +1,6 @@
 // Pieces shared by the solvers that keep one right-hand side's Krylov fields in
-// the registers and shared memory of a thread-block cluster (eo_cluster.cu).
+// the registers and shared memory of a thread-block cluster (eo_cluster.cu,
+// cg_cluster.cu).
 //
 // CTAs of a cluster exchange halo rows and partial sums by asynchronous remote
 // stores (st.async) that count their bytes on an mbarrier of the receiving CTA.
@@ -47,6 +48,13 @@ __device__ __forceinline__ void send(unsigned a, double v, unsigned bar)
 {
     asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(a),
                  "l"(__double_as_longlong(v)), "r"(bar)
+                 : "memory");
+}
+
+__device__ __forceinline__ void send(unsigned a, double2 v, unsigned bar)
+{
+    asm volatile("st.async.weak.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(a),
+                 "l"(__double_as_longlong(v.x)), "l"(__double_as_longlong(v.y)), "r"(bar)
                  : "memory");
 }
 
@@ -154,6 +162,66 @@ __device__ __forceinline__ void linger(unsigned long long limit_ns)
     const unsigned long long t0 = globaltimer_ns();
     while (globaltimer_ns() - t0 < 3 * limit_ns)
         __nanosleep(1000);
+}
+
+#define DWFB_SHFL_CPLX(T)                                                                        \
+    __device__ __forceinline__ T lane_c(T v, int src)                                          \
+    {                                                                                          \
+        return mkc(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));    \
+    }
+DWFB_SHFL_CPLX(float2)
+DWFB_SHFL_CPLX(double2)
+#undef DWFB_SHFL_CPLX
+
+// M5 v (M5^dag v when DAG: the part of D local in the 4-D site, diagonal and
+// fifth-dimension hop) for one 4-D site whose slices are spread over NL lanes at
+// distance 32 / NL, part q holding v[j], s = q LT + j (PAD: NL LT > Ls).
+template <bool DAG, bool PAD, int NL, typename R, int LT>
+__device__ __forceinline__ void m5(const Spinor<R> (&v)[LT], Spinor<R> (&o)[LT], int q, int Ls, R dg, R mf)
+{
+    using T = cplx<R>;
+    constexpr int D = 32 / NL;  // lanes between the parts of a site
+    const int lane = threadIdx.x & 31;
+    // spin component a(s) needs a(s+1), b(s) needs b(s-1)
+    auto a = [](const Spinor<R>& x) { return DAG ? x.s0 : x.s1; };
+    auto b = [](const Spinor<R>& x) { return DAG ? x.s1 : x.s0; };
+    const T up = lane_c(a(v[0]), (lane + D) & 31);       // next lane's first (wraps to s = 0)
+    T dn = lane_c(b(v[LT - 1]), (lane - D) & 31);        // previous lane's last
+    T first = up;
+    if (PAD)
+    {
+        const int ql = (Ls - 1) / LT, jl = Ls - 1 - ql * LT;
+        first = lane_c(a(v[0]), lane & (D - 1));
+        T last = b(v[0]);
+#pragma unroll
+        for (int j = 1; j < LT; ++j)
+            if (j == jl)
+                last = b(v[j]);
+        last = lane_c(last, D * ql + (lane & (D - 1)));
+        if (q == 0)
+            dn = last;
+    }
+#pragma unroll
+    for (int j = 0; j < LT; ++j)
+    {
+        const int s = q * LT + j;
+        const bool top = PAD ? s == Ls - 1 : (j == LT - 1 && q == NL - 1);
+        const T na = top ? first : (j + 1 < LT ? a(v[j + 1 < LT ? j + 1 : 0]) : up);
+        const T nb = j > 0 ? b(v[j > 0 ? j - 1 : 0]) : dn;
+        const R ca = top ? mf : R(-1), cb = (j == 0 && q == 0) ? mf : R(-1);
+        Spinor<R> r{dg * v[j].s0, dg * v[j].s1};
+        if (DAG)
+        {
+            r.s0 += ca * na;
+            r.s1 += cb * nb;
+        }
+        else
+        {
+            r.s1 += ca * na;
+            r.s0 += cb * nb;
+        }
+        o[j] = r;
+    }
 }
 
 }  // namespace cl

@@ -93,15 +93,6 @@ __device__ __forceinline__ float4 s2f4(const Spinor<float>& v)
     return make_float4(v.s0.x, v.s0.y, v.s1.x, v.s1.y);
 }
 
-#define DWFB_SHFL_CPLX(T)                                                                        \
-    __device__ __forceinline__ T lane_c(T v, int src)                                          \
-    {                                                                                          \
-        return mkc(__shfl_sync(0xffffffffu, v.x, src), __shfl_sync(0xffffffffu, v.y, src));    \
-    }
-DWFB_SHFL_CPLX(float2)
-DWFB_SHFL_CPLX(double2)
-#undef DWFB_SHFL_CPLX
-
 // The corner and carry weights of one lane's slices (q = the lane's part).
 template <typename R>
 struct M5w
@@ -148,14 +139,14 @@ __device__ __forceinline__ void cl_m5inv(Spinor<R> (&z)[LT], int q, const M5w<R>
 #pragma unroll
     for (int step = 1; step < NL; step *= 2)
     {
-        const T u = lane_c(B, (lane + step * D) & 31), v = lane_c(E, (lane - step * D) & 31);
+        const T u = cl::lane_c(B, (lane + step * D) & 31), v = cl::lane_c(E, (lane - step * D) & 31);
         B += cL * (q + step < NL ? u : zero);  // suffix scan
         E += cL * (q >= step ? v : zero);      // prefix scan
         cL *= cL;
     }
-    T cu = lane_c(B, (lane + D) & 31), cd = lane_c(E, (lane - D) & 31);
-    const T S = lane_c(B, lane & (D - 1));              // U(0)
-    T Sp = lane_c(E, (NL - 1) * D + (lane & (D - 1)));  // D(Ls-1), decayed by the padding
+    T cu = cl::lane_c(B, (lane + D) & 31), cd = cl::lane_c(E, (lane - D) & 31);
+    const T S = cl::lane_c(B, lane & (D - 1));              // U(0)
+    T Sp = cl::lane_c(E, (NL - 1) * D + (lane & (D - 1)));  // D(Ls-1), decayed by the padding
     if (PAD)
         Sp = w.pad * Sp;
     cu = (q + 1 < NL ? cu : zero) - w.qu * S;
@@ -173,55 +164,6 @@ __device__ __forceinline__ void cl_m5inv(Spinor<R> (&z)[LT], int q, const M5w<R>
             z[j].s1 += w.pw[LT - j] * cu;
             z[j].s0 += w.pw[j + 1] * cd;
         }
-    }
-}
-
-// M5 v (M5^dag v when DAG) for one 4-D site spread over its four lanes.
-template <bool DAG, bool PAD, int NL, int LT>
-__device__ __forceinline__ void cl_m5(const Spinor<float> (&v)[LT], Spinor<float> (&o)[LT], int q, int Ls,
-                                      float dg, float mf)
-{
-    constexpr int D = 32 / NL;
-    const int lane = threadIdx.x & 31;
-    // spin component a(s) needs a(s+1), b(s) needs b(s-1)
-    auto a = [](const Spinor<float>& x) { return DAG ? x.s0 : x.s1; };
-    auto b = [](const Spinor<float>& x) { return DAG ? x.s1 : x.s0; };
-    const float2 up = lane_c(a(v[0]), (lane + D) & 31);       // next lane's first (wraps to s = 0)
-    float2 dn = lane_c(b(v[LT - 1]), (lane - D) & 31);        // previous lane's last
-    float2 first = up;
-    if (PAD)
-    {
-        const int ql = (Ls - 1) / LT, jl = Ls - 1 - ql * LT;
-        first = lane_c(a(v[0]), lane & (D - 1));
-        float2 last = b(v[0]);
-#pragma unroll
-        for (int j = 1; j < LT; ++j)
-            if (j == jl)
-                last = b(v[j]);
-        last = lane_c(last, D * ql + (lane & (D - 1)));
-        if (q == 0)
-            dn = last;
-    }
-#pragma unroll
-    for (int j = 0; j < LT; ++j)
-    {
-        const int s = q * LT + j;
-        const bool top = PAD ? s == Ls - 1 : (j == LT - 1 && q == NL - 1);
-        const float2 na = top ? first : (j + 1 < LT ? a(v[j + 1 < LT ? j + 1 : 0]) : up);
-        const float2 nb = j > 0 ? b(v[j > 0 ? j - 1 : 0]) : dn;
-        const float ca = top ? mf : -1.f, cb = (j == 0 && q == 0) ? mf : -1.f;
-        Spinor<float> r{dg * v[j].s0, dg * v[j].s1};
-        if (DAG)
-        {
-            r.s0 += ca * na;
-            r.s1 += cb * nb;
-        }
-        else
-        {
-            r.s1 += ca * na;
-            r.s0 += cb * nb;
-        }
-        o[j] = r;
     }
 }
 
@@ -621,7 +563,8 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 for (int j = 0; j < LT; ++j)
                     p[j] = persist::axpy(beta, p[j], r[j]);
                 store(0, p);
-                __syncthreads();
+                if (__syncthreads_or(bad))
+                    break;
                 clk.mark(6);
                 // P1: y = M5^-1 H_eo p
                 halo(0);
@@ -653,7 +596,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     const ClLinks u = links(1);
                     const int ss = stride();
                     Spinor<float> m[LT];
-                    cl_m5<false, PAD, NL, LT>(p, m, q, Ls, dg, mf);
+                    cl::m5<false, PAD, NL>(p, m, q, Ls, dg, mf);
                     if (on)
 #pragma unroll
                         for (int j = 0; j < LT; ++j)
@@ -712,7 +655,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
 #pragma unroll
                     for (int j = 0; j < LT; ++j)
                         tv[j] = act(j) ? f4s(FA[(s0 + j) * ss + own]) : zero;
-                    cl_m5<true, PAD, NL, LT>(tv, m, q, Ls, dg, mf);
+                    cl::m5<true, PAD, NL>(tv, m, q, Ls, dg, mf);
                     if (on)
 #pragma unroll
                         for (int j = 0; j < LT; ++j)
@@ -735,8 +678,6 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     sum.send(0);
                 clk.mark(4);
                 const double rn = total(0);
-                if (__syncthreads_or(bad))
-                    break;
                 want = rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
                 cf = rn / rr;
                 rr = rn;

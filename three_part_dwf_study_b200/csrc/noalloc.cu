@@ -19,6 +19,7 @@
 #include <algorithm>
 #include <mutex>
 
+#include "cg_cluster.cuh"
 #include "context.cuh"
 #include "kernels.cuh"
 #include "single.cuh"
@@ -170,7 +171,9 @@ extern "C" int dwf_cg_noalloc(const dwf_params* p, int op, const double* theta_d
     if (single_part_doubles(nsm) > size_t(kPartDoubles))
         return DWF_CUDA_ERROR;
     d.part = part;
-    if (launch_single(d, false, nsm, stream) != cudaSuccess)
+    bool clustered = false;
+    if (launch_cg_cluster(d, false, p->device, nsm, stream, &clustered) != cudaSuccess ||
+        (!clustered && launch_single(d, false, nsm, stream) != cudaSuccess))
         return DWF_CUDA_ERROR;
 
     // FP64 true residual |b - A x| / |b| with the scratch temporary t
