@@ -969,26 +969,72 @@ struct GradArgs
     float2* part;  // [gridDim.x][9][cout][cin]
 };
 
-constexpr int kGradSites = 32;
-constexpr int kGradThreads = 256;
-// weights per thread: cout * cin <= kGradThreads * PER; 4 for layers up to
-// 1024 complex weights per offset, 6 up to 1536 (48 x 32: Ls = 24, 32 hidden)
-constexpr int kGradMaxPer = 6;
+constexpr int kGradSites = 16;
+constexpr int kGradSmem = 96 * 1024;  // most a layer's stage needs (48 x 32: 60 KB)
+constexpr int kGradMaxWeights = 1536;  // complex weights per offset (48 x 32: Ls = 24, 32 hidden)
 
-template <int PER>
-__global__ void __launch_bounds__(kGradThreads) lp_wgrad_kernel(GradArgs a)
+// Shape of a layer's weight gradient: 4 x 4 tiles of (output, input) channels, one
+// thread per offset, tile and share of a chunk's sites.
+struct GradShape
 {
-    constexpr int kGradMaxPer = PER;
+    int OT, IT;   // tiles of output and input channels
+    int split;    // threads that share one tile's sites
+    int width;    // lanes per row while staging (a power of two)
+    int threads;  // 9 OT IT split, rounded to warps
+    size_t smem;
+};
+
+__host__ inline GradShape grad_shape(int cin, int cout)
+{
+    GradShape g;
+    g.OT = (cout + 3) / 4;
+    g.IT = (cin + 3) / 4;
+    const int tiles = 9 * g.OT * g.IT;
+    g.split = 1;
+    while (g.split < 8 && tiles * g.split * 2 <= 576)
+        g.split *= 2;
+    g.threads = (tiles * g.split + 31) / 32 * 32;
+    g.width = 4;
+    while (g.width < 32 && g.width < 4 * (g.OT > g.IT ? g.OT : g.IT))
+        g.width *= 2;
+    const size_t stage = size_t(kGradSites) * 4 * (g.OT + 9 * g.IT) * sizeof(float2);
+    const size_t sums = size_t(g.split > 1 ? g.split : 0) * tiles * 16 * sizeof(float2);
+    g.smem = stage > sums ? stage : sums;
+    return g;
+}
+
+// Per chunk of 16 sites of one field the block stages g and, for every offset, the
+// transported BF16 input a_k, then each thread adds its 4 x 4 tile's 16 complex
+// products per site from four 16-byte shared loads. (One weight per thread and
+// offset loaded 16 bytes for four multiply-adds and was bound by those loads:
+// 32 x 32 weights, 8 fields of 64x64 sites 241 us a layer, now 103; the FP32 pipes'
+// time is 32. Rows of lanes instead of a division per staged element took 185 to
+// 128, four multiply-adds a product instead of six operations 128 to 103; staging,
+// which alternates with the products, and its gathers are what is left.) Channels 4i, 4i+1 and 4i+2, 4i+3 of the tiles i lie
+// in two planes, so that a warp's 16-byte loads touch consecutive words. Small
+// layers leave threads for several shares of the sites, added at the end.
+template <int MAXT, int MINB>
+__global__ void __launch_bounds__(MAXT, MINB) lp_wgrad_kernel(GradArgs a, GradShape gs)
+{
     extern __shared__ __align__(16) unsigned char smem[];
-    float2* gs = reinterpret_cast<float2*>(smem);      // [32][cout]
-    float2* as = gs + kGradSites * a.cout;             // [32][cin]
-    const int E = a.cout * a.cin;
-    float2 acc[9][kGradMaxPer];
+    float2* const G = reinterpret_cast<float2*>(smem);  // [site][plane][OT][2]
+    float2* const A = G + kGradSites * 4 * gs.OT;       // [offset][site][plane][IT][2]
+    const int tiles = gs.OT * gs.IT, nt = 9 * tiles;
+    const int sp = threadIdx.x / nt, e0 = threadIdx.x - sp * nt;
+    const int k = e0 / tiles, tile = e0 - k * tiles;
+    const int oi = tile / gs.IT, ii = tile - oi * gs.IT;
+    const bool on = sp < gs.split;
+    float2 acc[4][4];
 #pragma unroll
-    for (int k = 0; k < 9; ++k)
+    for (int o = 0; o < 4; ++o)
 #pragma unroll
-        for (int m = 0; m < kGradMaxPer; ++m)
-            acc[k][m] = make_float2(0.f, 0.f);
+        for (int i = 0; i < 4; ++i)
+            acc[o][i] = make_float2(0.f, 0.f);
+    const int ci4 = 4 * gs.IT, co4 = 4 * gs.OT;
+    __shared__ int NB[9 * kGradSites];
+    __shared__ float2 TR[9 * kGradSites];
+    const int width = gs.width, rows = int(blockDim.x) / width;
+    const int col0 = threadIdx.x & (width - 1), row0 = int(threadIdx.x) / width;
     const int chunks_per_rhs = (a.V + kGradSites - 1) / kGradSites;
     const long nchunks = long(chunks_per_rhs) * a.nrhs;
     for (long chn = blockIdx.x; chn < nchunks; chn += gridDim.x)
@@ -996,88 +1042,140 @@ __global__ void __launch_bounds__(kGradThreads) lp_wgrad_kernel(GradArgs a)
         const int rhs = int(chn / chunks_per_rhs);
         const int h0 = int(chn - long(rhs) * chunks_per_rhs) * kGradSites;
         const int cf = a.conf ? a.conf[rhs] : a.conf0;
-        const float2* Tc = a.T + long(cf) * a.V * 9;
-        const float2* inr = a.in + long(rhs) * a.li.rs;
-        const float2* gr = a.g + long(rhs) * a.lg.rs;
+        const float2* const Tc = a.T + long(cf) * a.V * 9;
+        const float2* const inr = a.in + long(rhs) * a.li.rs;
+        const float2* const gr = a.g + long(rhs) * a.lg.rs;
         __syncthreads();
-        for (int e = threadIdx.x; e < kGradSites * a.cout; e += blockDim.x)
+        // where each (offset, site) row's input lies, and its transporter
+        for (int e = threadIdx.x; e < 9 * kGradSites; e += blockDim.x)
         {
-            const int r = e / a.cout, o = e - r * a.cout;
-            const int h = h0 + r;
-            gs[e] = (h < a.V) ? gr[long(h) * a.lg.hs + chan_off(a.lg, o)] : make_float2(0.f, 0.f);
-        }
-#pragma unroll
-        for (int k = 0; k < 9; ++k)
-        {
-            __syncthreads();
-            for (int e = threadIdx.x; e < kGradSites * a.cin; e += blockDim.x)
+            const int kk = e / kGradSites, h = h0 + e - kk * kGradSites;
+            int nb = -1;
+            float2 T = make_float2(0.f, 0.f);
+            if (h < a.V)
             {
-                const int r = e / a.cin, i = e - r * a.cin;
+                const int t = h / a.Nx, x = h - t * a.Nx;
+                int tt = t + kOffT[kk], xx = x + kOffX[kk];
+                tt = tt < 0 ? tt + a.Nt : (tt >= a.Nt ? tt - a.Nt : tt);
+                xx = xx < 0 ? xx + a.Nx : (xx >= a.Nx ? xx - a.Nx : xx);
+                nb = tt * a.Nx + xx;
+                T = Tc[long(h) * 9 + kk];
+            }
+            NB[e] = nb;
+            TR[e] = T;
+        }
+        __syncthreads();
+        // rows of `width` lanes: no division per element
+        for (int r = row0; r < kGradSites; r += rows)
+            for (int o = col0; o < co4; o += width)
+            {
                 const int h = h0 + r;
+                G[((r * 2 + ((o >> 1) & 1)) * gs.OT + (o >> 2)) * 2 + (o & 1)] =
+                    (h < a.V && o < a.cout) ? gr[long(h) * a.lg.hs + chan_off(a.lg, o)] : make_float2(0.f, 0.f);
+            }
+        for (int i = col0; i < ci4; i += width)
+        {
+            const float2* const src = inr + (i < a.cin ? chan_off(a.li, i) : 0);
+            float2* const dst = A + ((((i >> 1) & 1) * gs.IT) + (i >> 2)) * 2 + (i & 1);
+#pragma unroll 4
+            for (int kr = row0; kr < 9 * kGradSites; kr += rows)
+            {
+                const int nb = NB[kr];
                 float2 v = make_float2(0.f, 0.f);
-                if (h < a.V)
+                if (nb >= 0 && i < a.cin)
                 {
-                    const int t = h / a.Nx, x = h - t * a.Nx;
-                    int tt = t + kOffT[k], xx = x + kOffX[k];
-                    tt = tt < 0 ? tt + a.Nt : (tt >= a.Nt ? tt - a.Nt : tt);
-                    xx = xx < 0 ? xx + a.Nx : (xx >= a.Nx ? xx - a.Nx : xx);
-                    const float2 T = Tc[long(h) * 9 + k];
-                    const float2 u = inr[long(tt * a.Nx + xx) * a.li.hs + chan_off(a.li, i)];
+                    const float2 T = TR[kr], u = src[long(nb) * a.li.hs];
                     const uint32_t b = pack_bf2(u.x, u.y);
                     const float2 ub = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&b));
                     v = make_float2(T.x * ub.x - T.y * ub.y, T.x * ub.y + T.y * ub.x);
                 }
-                as[e] = v;
+                dst[kr * 4 * gs.IT] = v;
             }
-            __syncthreads();
-#pragma unroll
-            for (int m = 0; m < kGradMaxPer; ++m)
+        }
+        __syncthreads();
+        if (on)
+        {
+            const float4* const G4 = reinterpret_cast<const float4*>(G) + oi;
+            const float4* const A4 = reinterpret_cast<const float4*>(A) + long(k) * kGradSites * 2 * gs.IT + ii;
+            for (int r = sp; r < kGradSites; r += gs.split)
             {
-                const int e = threadIdx.x + m * kGradThreads;
-                if (e < E)
-                {
-                    const int o = e / a.cin, i = e - o * a.cin;
-                    float2 s = acc[k][m];
-                    for (int r = 0; r < kGradSites; ++r)
+                const float4 g0 = G4[r * 2 * gs.OT], g1 = G4[(r * 2 + 1) * gs.OT];
+                const float4 a0 = A4[r * 2 * gs.IT], a1 = A4[(r * 2 + 1) * gs.IT];
+                const float2 gv[4] = {{g0.x, g0.y}, {g0.z, g0.w}, {g1.x, g1.y}, {g1.z, g1.w}};
+                const float2 av[4] = {{a0.x, a0.y}, {a0.z, a0.w}, {a1.x, a1.y}, {a1.z, a1.w}};
+#pragma unroll
+                for (int o = 0; o < 4; ++o)
+#pragma unroll
+                    for (int i = 0; i < 4; ++i)
                     {
-                        const float2 gv = gs[r * a.cout + o];
-                        const float2 av = as[r * a.cin + i];
-                        // g * conj(a)
-                        s.x += gv.x * av.x + gv.y * av.y;
-                        s.y += gv.y * av.x - gv.x * av.y;
+                        // g * conj(a), four multiply-adds (as one sum each, six operations)
+                        acc[o][i].x = fmaf(gv[o].x, av[i].x, acc[o][i].x);
+                        acc[o][i].y = fmaf(gv[o].y, av[i].x, acc[o][i].y);
+                        acc[o][i].x = fmaf(gv[o].y, av[i].y, acc[o][i].x);
+                        acc[o][i].y = fmaf(-gv[o].x, av[i].y, acc[o][i].y);
                     }
-                    acc[k][m] = s;
-                }
             }
         }
     }
-    float2* p = a.part + long(blockIdx.x) * 9 * E;
+    float2* const p = a.part + long(blockIdx.x) * 9 * a.cout * a.cin;
+    if (gs.split > 1)
+    {
+        float2* const S = reinterpret_cast<float2*>(smem);  // [split][9 tiles][16]
+        __syncthreads();
+        if (on)
 #pragma unroll
-    for (int k = 0; k < 9; ++k)
+            for (int o = 0; o < 4; ++o)
 #pragma unroll
-        for (int m = 0; m < kGradMaxPer; ++m)
-        {
-            const int e = threadIdx.x + m * kGradThreads;
-            if (e < E)
-                p[k * E + e] = acc[k][m];
-        }
+                for (int i = 0; i < 4; ++i)
+                    S[(sp * nt + e0) * 16 + o * 4 + i] = acc[o][i];
+        __syncthreads();
+        if (sp != 0)
+            return;
+#pragma unroll
+        for (int o = 0; o < 4; ++o)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                for (int q = 1; q < gs.split; ++q)
+                    acc[o][i] += S[(q * nt + e0) * 16 + o * 4 + i];
+    }
+    if (sp == 0)
+#pragma unroll
+        for (int o = 0; o < 4; ++o)
+#pragma unroll
+            for (int i = 0; i < 4; ++i)
+                if (4 * oi + o < a.cout && 4 * ii + i < a.cin)
+                    p[(long(k) * a.cout + 4 * oi + o) * a.cin + 4 * ii + i] = acc[o][i];
 }
 
-// grad[e] = sum over blocks of part[b][e], in FP64 and block order.
-__global__ void lp_grad_reduce_kernel(const float2* __restrict__ part, int nblk, int n,
-                                      float2* __restrict__ grad)
+// grad[e] = sum over blocks of part[b][e], in FP64: eight threads per weight take
+// every eighth block in order, their sums are added in order (one thread per weight
+// walked all blocks: 19 us for 9216 weights, now 13).
+constexpr int kGradReduce = 8;
+__global__ void __launch_bounds__(256) lp_grad_reduce_kernel(const float2* __restrict__ part, int nblk, int n,
+                                                             float2* __restrict__ grad)
 {
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n; e += gridDim.x * blockDim.x)
-    {
-        double sx = 0.0, sy = 0.0;
-        for (int b = 0; b < nblk; ++b)
+    __shared__ double2 sm[kGradReduce][32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    const int e = blockIdx.x * 32 + lane;
+    double sx = 0.0, sy = 0.0;
+    if (e < n)
+#pragma unroll 8
+        for (int b = w; b < nblk; b += kGradReduce)
         {
             const float2 v = part[long(b) * n + e];
             sx += v.x;
             sy += v.y;
         }
-        grad[e] = make_float2(float(sx), float(sy));
+    sm[w][lane] = make_double2(sx, sy);
+    __syncthreads();
+    if (w != 0 || e >= n)
+        return;
+    for (int q = 1; q < kGradReduce; ++q)
+    {
+        sx += sm[q][lane].x;
+        sy += sm[q][lane].y;
     }
+    grad[e] = make_float2(float(sx), float(sy));
 }
 
 // ---------------------------------------------------------------------------
@@ -2397,13 +2495,17 @@ int lp_loss_grad(dwf_ctx* c, int nrhs, const int* conf_d, const float2* rho, con
         a.V = c->L.V;
         a.nrhs = nrhs;
         a.part = n->gpart;
-        const size_t smem = size_t(kGradSites) * (a.cin + a.cout) * sizeof(float2);
-        if (a.cin * a.cout <= kGradThreads * 4)
-            lp_wgrad_kernel<4><<<nblk_g, kGradThreads, smem, c->stream>>>(a);
+        const GradShape gs = grad_shape(a.cin, a.cout);
+        const bool wide = gs.threads > 576;
+        const void* fn = wide ? reinterpret_cast<const void*>(&lp_wgrad_kernel<864, 1>)
+                              : reinterpret_cast<const void*>(&lp_wgrad_kernel<576, 2>);
+        CK(cudaFuncSetAttribute(fn, cudaFuncAttributeMaxDynamicSharedMemorySize, kGradSmem));
+        if (wide)
+            lp_wgrad_kernel<864, 1><<<nblk_g, gs.threads, gs.smem, c->stream>>>(a, gs);
         else
-            lp_wgrad_kernel<kGradMaxPer><<<nblk_g, kGradThreads, smem, c->stream>>>(a);
+            lp_wgrad_kernel<576, 2><<<nblk_g, gs.threads, gs.smem, c->stream>>>(a, gs);
         const int E = 9 * a.cin * a.cout;
-        lp_grad_reduce_kernel<<<(E + 255) / 256, 256, 0, c->stream>>>(n->gpart, nblk_g, E, n->G + n->woff[l]);
+        lp_grad_reduce_kernel<<<(E + 31) / 32, 256, 0, c->stream>>>(n->gpart, nblk_g, E, n->G + n->woff[l]);
         c->launches += 2;
         CK(cudaGetLastError());
         if (l > 0)
@@ -3057,7 +3159,7 @@ int dwf_lp_init(dwf_ctx* c, int hidden, uint64_t seed)
     if (hidden != 8 && hidden != 16 && hidden != 24 && hidden != 32)
         return ctx_fail(c, DWF_BAD_ARG, "dwf_lp_init: hidden must be 8, 16, 24 or 32");
     const int C0 = 2 * c->L.Ls;
-    if (C0 > 48 || C0 * hidden > kGradThreads * kGradMaxPer)
+    if (C0 > 48 || C0 * hidden > kGradMaxWeights)
         return ctx_fail(c, DWF_BAD_ARG, "dwf_lp_init: 2*Ls*hidden must be <= 1536 and Ls <= 24");
     CK(cudaSetDevice(c->device));
     lp_destroy(c);
