@@ -192,7 +192,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
     for (int it = 1; it <= d.maxiter && nact > 0; ++it)
     {
         // P1: y = M5^-1 H_eo p
-        sweep_sites(d, s.act, nact, nsite4, e.nch4, e.ch4, s.scratch, false,
+        sweep_sites(d, s.act, nact, nsite4, e.nch4, e.ch4, s.scratch, 0,
                     [&](int j, int h, long uo) {
                         const int t = h / g.Nxh, k = h - t * g.Nxh;
                         if (e.zsmem)
@@ -209,7 +209,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
             return;
         phase_mark(e.phase_ns, 0, ph_t);
         // P2: t = M5 p - H_oe y, |t|^2
-        sweep_sites(d, s.act, nact, nsite5, d.nch, d.ch, s.scratch, true,
+        sweep_sites(d, s.act, nact, nsite5, d.nch, d.ch, s.scratch, kSlot0,
                     [&](int j, int i, long uo) {
                         const int ss = i / g.Vh, h = i - ss * g.Vh;
                         const Spinor<float> v = eo_combine_site<false, float>(
@@ -238,7 +238,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
         nact = compact(d.nrhs, s.act, s.scratch, [&](int j) { return s.state[j] == RHS_ACTIVE; });
         phase_mark(e.phase_ns, 2, ph_t);
         // P3: y = M5^dag^-1 H^dag_eo t
-        sweep_sites(d, s.act, nact, nsite4, e.nch4, e.ch4, s.scratch, false,
+        sweep_sites(d, s.act, nact, nsite4, e.nch4, e.ch4, s.scratch, 0,
                     [&](int j, int h, long uo) {
                         const int t = h / g.Nxh, k = h - t * g.Nxh;
                         if (e.zsmem)
@@ -255,7 +255,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
             return;
         phase_mark(e.phase_ns, 3, ph_t);
         // P4: Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap
-        sweep_sites(d, s.act, nact, nsite5, d.nch, d.ch, s.scratch, true,
+        sweep_sites(d, s.act, nact, nsite5, d.nch, d.ch, s.scratch, kSlot0,
                     [&](int j, int i, long uo) {
                         const int ss = i / g.Vh, h = i - ss * g.Vh;
                         const float a = float(s.al[j]);
@@ -295,7 +295,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
         {
             // FP64 residual of the Schur normal equation at x + e:
             // (a) y64 = M5^-1 H_eo (x + e)
-            sweep_sites(d, s.act, nru, nsite4, e.nch4, e.ch4, s.scratch, false,
+            sweep_sites(d, s.act, nru, nsite4, e.nch4, e.ch4, s.scratch, 0,
                         [&](int j, int h, long uo) {
                             const int t = h / g.Nxh, k = h - t * g.Nxh;
                             eo_hopinv_site<false, double>(SumLd{d.x + j * fh, d.e32 + j * fh},
@@ -306,7 +306,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
             if (!grid_sync(d.bar, d.expected_blocks, d.timeout_ns))
                 return;
             // (b) t64 = M5 (x + e) - H_oe y64; park x + e in xn64
-            sweep_sites(d, s.act, nru, nsite5, d.nch, d.ch, s.scratch, false,
+            sweep_sites(d, s.act, nru, nsite5, d.nch, d.ch, s.scratch, 0,
                         [&](int j, int i, long uo) {
                             const int ss = i / g.Vh, h = i - ss * g.Vh;
                             const SumLd xe{d.x + j * fh, d.e32 + j * fh};
@@ -320,7 +320,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
             if (!grid_sync(d.bar, d.expected_blocks, d.timeout_ns))
                 return;
             // (c) y64 = M5^dag^-1 H^dag_eo t64
-            sweep_sites(d, s.act, nru, nsite4, e.nch4, e.ch4, s.scratch, false,
+            sweep_sites(d, s.act, nru, nsite4, e.nch4, e.ch4, s.scratch, 0,
                         [&](int j, int h, long uo) {
                             const int t = h / g.Nxh, k = h - t * g.Nxh;
                             eo_hopinv_site<true, double>(FieldLd<double>{d.t + j * fh}, true,
@@ -331,7 +331,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
             if (!grid_sync(d.bar, d.expected_blocks, d.timeout_ns))
                 return;
             // (d) r = b - (M5^dag t64 - H^dag_oe y64); x = x + e; r32 = r; e = 0
-            sweep_sites(d, s.act, nru, nsite5, d.nch, d.ch, s.scratch, true,
+            sweep_sites(d, s.act, nru, nsite5, d.nch, d.ch, s.scratch, kSlot0,
                         [&](int j, int i, long uo) {
                             const int ss = i / g.Vh, h = i - ss * g.Vh;
                             const Spinor<double> a = eo_combine_site<true, double>(
@@ -372,7 +372,7 @@ __global__ void __launch_bounds__(256, DWFB_EO_MINB) cg_eo_mixed_kernel(EoDesc e
             break;
         phase_mark(e.phase_ns, 5, ph_t);
         // P5: p = r + beta p
-        sweep_sites(d, s.act, nact, nsite5, d.nch, d.ch, s.scratch, false,
+        sweep_sites(d, s.act, nact, nsite5, d.nch, d.ch, s.scratch, 0,
                     [&](int j, int i, long uo) {
                         const Spinor<float> p = ld_spinor(d.p32 + j * fh, i);
                         const Spinor<float> r = ld_spinor(d.r32 + j * fh, i);

@@ -102,10 +102,15 @@ __device__ inline void reduce_listed(const SolveDesc& d, const int* act, int nac
 
 // Visit sites [0, nsite) of every listed right-hand side in units of `ch`
 // sites (nch units per right-hand side); f(j, i, uo) returns two partial-sum
-// contributions, stored per unit when `keep` is set (uo: the unit's link offset).
+// contributions, of which those in the mask `keep` (kSlot0, kSlot1) are stored per
+// unit (uo: the unit's link offset). A block reads the partials of every unit
+// after the grid barrier while a faster block may already be in its next sweep,
+// so two sweeps with one barrier between them must keep different slots.
+constexpr int kSlot0 = 1, kSlot1 = 2;
+
 template <typename F>
 __device__ void sweep_sites(const SolveDesc& d, const int* act, int nact, int nsite, int nch,
-                            int ch, double* scratch, bool keep, F f)
+                            int ch, double* scratch, int keep, F f)
 {
     const int nunits = nact * nch;
     for (int u = blockIdx.x; u < nunits; u += gridDim.x)
@@ -122,22 +127,24 @@ __device__ void sweep_sites(const SolveDesc& d, const int* act, int nact, int ns
             a0 += v.x;
             a1 += v.y;
         }
-        if (keep)
+        if (keep & kSlot0)
         {
             a0 = block_sum(a0, scratch);
+            if (threadIdx.x == 0)
+                d.part[(long(j) * nch + c) * 2] = a0;
+        }
+        if (keep & kSlot1)
+        {
             a1 = block_sum(a1, scratch);
             if (threadIdx.x == 0)
-            {
-                d.part[(long(j) * nch + c) * 2] = a0;
                 d.part[(long(j) * nch + c) * 2 + 1] = a1;
-            }
         }
     }
 }
 
 // The full-lattice sweep (nsite = Ls*V, the launch's chunking).
 template <typename F>
-__device__ void sweep(const SolveDesc& d, const int* act, int nact, double* scratch, bool keep,
+__device__ void sweep(const SolveDesc& d, const int* act, int nact, double* scratch, int keep,
                       F f)
 {
     sweep_sites(d, act, nact, d.L.nsite, d.nch, d.ch, scratch, keep, f);
@@ -222,7 +229,7 @@ __device__ inline bool init_residual(const SolveDesc& d, const Smem& s, int nact
     const bool dag1 = d.dag_first != 0;
     if (d.has_guess)
     {
-        sweep(d, s.act, nact, s.scratch, false, [&](int j, int i, long uo) {
+        sweep(d, s.act, nact, s.scratch, 0, [&](int j, int i, long uo) {
             const Spinor<double> v = op_site<double>(d, dag1, d.x + j * fs, d.U64 + uo, i);
             st_spinor(d.t + j * fs, i, v);
             return make_double2(0.0, 0.0);
@@ -230,7 +237,7 @@ __device__ inline bool init_residual(const SolveDesc& d, const Smem& s, int nact
         if (!grid_sync(d.bar, d.expected_blocks, d.timeout_ns))
             return false;
     }
-    sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
+    sweep(d, s.act, nact, s.scratch, kSlot0 | kSlot1, [&](int j, int i, long uo) {
         const Spinor<double> b = ld_spinor(d.b + j * fs, i);
         Spinor<double> r = b;
         if (d.has_guess)
@@ -257,7 +264,8 @@ __device__ inline bool init_residual(const SolveDesc& d, const Smem& s, int nact
         return false;
     reduce_listed(d, s.act, nact, 0, s.bb);
     reduce_listed(d, s.act, nact, 1, s.rr);
-    return true;
+    // the first sweep of the iteration stores into the slots just read
+    return grid_sync(d.bar, d.expected_blocks, d.timeout_ns);
 }
 
 // Initial convergence test (cg_solver.hpp:30-38; Eigen rule: |r|^2 < tol^2 |b|^2).

@@ -53,7 +53,7 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
     for (int it = 1; it <= d.maxiter && nact > 0; ++it)
     {
         // phase 1: t = D1 p, <p, A p> = |t|^2
-        sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
+        sweep(d, s.act, nact, s.scratch, kSlot0, [&](int j, int i, long uo) {
             const Spinor<double> v = op_site<double>(d, dag1, d.p + j * fs, d.U64 + uo, i);
             st_spinor(d.t + j * fs, i, v);
             return make_double2(spinor_norm2(v), 0.0);
@@ -76,7 +76,7 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
         nact = compact(d.nrhs, s.act, s.scratch, [&](int j) { return s.state[j] == RHS_ACTIVE; });
 
         // phase 2: x += alpha p; r -= alpha A p
-        sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
+        sweep(d, s.act, nact, s.scratch, kSlot1, [&](int j, int i, long uo) {
             const double a = s.al[j];
             const Spinor<double> ap = op_site<double>(d, !dag1, d.t + j * fs, d.U64 + uo, i);
             const Spinor<double> p = ld_spinor(d.p + j * fs, i);
@@ -85,11 +85,11 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
             st_spinor(d.x + j * fs, i, axpy(a, p, x));
             const Spinor<double> rn = axpy(-a, ap, r);
             st_spinor(d.r + j * fs, i, rn);
-            return make_double2(spinor_norm2(rn), 0.0);
+            return make_double2(0.0, spinor_norm2(rn));
         });
         if (!grid_sync(d.bar, d.expected_blocks, d.timeout_ns))
             return;
-        reduce_listed(d, s.act, nact, 0, s.aux);
+        reduce_listed(d, s.act, nact, 1, s.aux);
         for (int k = threadIdx.x; k < nact; k += blockDim.x)
         {
             const int j = s.act[k];
@@ -112,7 +112,7 @@ __global__ void __launch_bounds__(256, MINB) cg64_kernel(SolveDesc d)
         if (nact == 0)
             break;
         // phase 3: p = r + beta p
-        sweep(d, s.act, nact, s.scratch, false, [&](int j, int i, long uo) {
+        sweep(d, s.act, nact, s.scratch, 0, [&](int j, int i, long uo) {
             const Spinor<double> p = ld_spinor(d.p + j * fs, i);
             const Spinor<double> r = ld_spinor(d.r + j * fs, i);
             st_spinor(d.p + j * fs, i, axpy(s.cf[j], p, r));
@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
     // stall counters live in the upper bits of flag: flag = 2*stalls + update bit
     for (int it = 1; it <= d.maxiter && nact > 0; ++it)
     {
-        sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
+        sweep(d, s.act, nact, s.scratch, kSlot0, [&](int j, int i, long uo) {
             const Spinor<float> v = op_site<float>(d, dag1, d.p32 + j * fs, d.U32 + uo, i);
             st_spinor(d.t32 + j * fs, i, v);
             return make_double2(spinor_norm2(v), 0.0);
@@ -182,7 +182,7 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
         __syncthreads();
         nact = compact(d.nrhs, s.act, s.scratch, [&](int j) { return s.state[j] == RHS_ACTIVE; });
 
-        sweep(d, s.act, nact, s.scratch, true, [&](int j, int i, long uo) {
+        sweep(d, s.act, nact, s.scratch, kSlot1, [&](int j, int i, long uo) {
             const float a = float(s.al[j]);
             const Spinor<float> ap = op_site<float>(d, !dag1, d.t32 + j * fs, d.U32 + uo, i);
             const Spinor<float> p = ld_spinor(d.p32 + j * fs, i);
@@ -191,11 +191,11 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
             st_spinor(d.e32 + j * fs, i, axpy(a, p, e));
             const Spinor<float> rn = axpy(-a, ap, r);
             st_spinor(d.r32 + j * fs, i, rn);
-            return make_double2(spinor_norm2(rn), 0.0);
+            return make_double2(0.0, spinor_norm2(rn));
         });
         if (!grid_sync(d.bar, d.expected_blocks, d.timeout_ns))
             return;
-        reduce_listed(d, s.act, nact, 0, s.aux);
+        reduce_listed(d, s.act, nact, 1, s.aux);
         for (int k = threadIdx.x; k < nact; k += blockDim.x)
         {
             const int j = s.act[k];
@@ -216,7 +216,7 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
         {
             // Reliable update, part 1: t = D1 (x + e) in FP64, with x + e
             // formed on the fly from its neighbourhood and parked in r.
-            sweep(d, s.act, nru, s.scratch, false, [&](int j, int i, long uo) {
+            sweep(d, s.act, nru, s.scratch, 0, [&](int j, int i, long uo) {
                 int ss, tt, xx;
                 site_coords(d.L, i, ss, tt, xx);
                 const SumLd xe{d.x + j * fs, d.e32 + j * fs};
@@ -230,7 +230,7 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
             if (!grid_sync(d.bar, d.expected_blocks, d.timeout_ns))
                 return;
             // part 2: x = x + e; r = b - D2 t; r32 = r; e = 0
-            sweep(d, s.act, nru, s.scratch, true, [&](int j, int i, long uo) {
+            sweep(d, s.act, nru, s.scratch, kSlot0, [&](int j, int i, long uo) {
                 const Spinor<double> xn = ld_spinor(d.r + j * fs, i);
                 const Spinor<double> a = op_site<double>(d, !dag1, d.t + j * fs, d.U64 + uo, i);
                 const Spinor<double> b = ld_spinor(d.b + j * fs, i);
@@ -266,7 +266,7 @@ __global__ void __launch_bounds__(256, MINB) cg_mixed_kernel(SolveDesc d)
         nact = compact(d.nrhs, s.act, s.scratch, [&](int j) { return s.state[j] == RHS_ACTIVE; });
         if (nact == 0)
             break;
-        sweep(d, s.act, nact, s.scratch, false, [&](int j, int i, long uo) {
+        sweep(d, s.act, nact, s.scratch, 0, [&](int j, int i, long uo) {
             const Spinor<float> p = ld_spinor(d.p32 + j * fs, i);
             const Spinor<float> r = ld_spinor(d.r32 + j * fs, i);
             st_spinor(d.p32 + j * fs, i, axpy(float(s.cf[j]), p, r));
