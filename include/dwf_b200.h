@@ -362,8 +362,8 @@ int dwf_barrier_selftest(dwf_ctx* ctx, int missing_blocks, uint64_t limit_ns);
  * Ls <= 16; else as 0), 4 = Wilson contexts only: one thread per four
  * consecutive rows of one column, all loads up front into registers (Nx a
  * multiple of 32 and Nt of 4; else as 0), 5 = as 1 with the x neighbours
- * exchanged by warp shuffles and the next slice's loads issued ahead (Nx a
- * multiple of 32; else as 1), 6 = as 1 with each block's slices (its 32 x 8
+ * exchanged by warp shuffles and the next slice's loads issued ahead (warps
+ * along a row where Nx is a multiple of 32, along the flattened plane else), 6 = as 1 with each block's slices (its 32 x 8
  * sites and their halo) brought into a shared-memory ring by 1-D bulk copies
  * completing on mbarriers, every neighbour read from shared memory (Nx a
  * multiple of 32 and Nt of 8; else as 0; chosen only by this call: slower

@@ -301,6 +301,14 @@ void launch_dirac(dwf_ctx* c, DslashChoice ch, bool dag, int nrhs, const int* co
         prefer_l1(c, 0 + (dag ? 1 : 0) + (sizeof(R) == 8 ? 2 : 0), kern);
         kern<<<grid, 256, 0, c->stream>>>(c->L, in, out, fs, U, c->usz(), conf_d, conf0);
     }
+    else if (variant == 5)
+    {
+        // a row's lanes would be ragged: the flattened column kernel
+        const dim3 grid((c->L.V + 127) / 128, nrhs);
+        auto kern = dag ? dirac_colf_kernel<true, R> : dirac_colf_kernel<false, R>;
+        prefer_l1(c, 16 + (dag ? 1 : 0) + (sizeof(R) == 8 ? 2 : 0), kern);
+        kern<<<grid, 128, 0, c->stream>>>(c->L, in, out, fs, U, c->usz(), conf_d, conf0);
+    }
     else if (variant == 6 && tile_ok(c->L) && c->dslash_err)
     {
         const dim3 grid(c->L.Nx / 32, c->L.Nt / kRingT, nrhs);
@@ -322,7 +330,7 @@ void launch_dirac(dwf_ctx* c, DslashChoice ch, bool dag, int nrhs, const int* co
         kern<<<grid, 256, tile_smem_bytes(2 * sizeof(cplx<R>)), c->stream>>>(
             c->L, in, out, fs, U, c->usz(), conf_d, conf0, c->dslash_err, c->timeout_ns);
     }
-    else if (variant == 1 || variant == 5)
+    else if (variant == 1)
     {
         const dim3 grid((c->L.Nx + 31) / 32, (c->L.Nt + 7) / 8, nrhs);
         auto kern = dag ? dirac_col_kernel<true, R> : dirac_col_kernel<false, R>;
@@ -353,13 +361,15 @@ void launch_dirac(dwf_ctx* c, DslashChoice ch, bool dag, int nrhs, const int* co
     c->launches += 1;
 }
 
+// (On ragged rows the flattened form of 5 was as fast as 1 or faster wherever timed,
+// so 1 is no candidate there.)
 // Autotuner: time the variants (two applications each, CUDA events on the
 // context stream) for this precision and batch-size bucket, keep the fastest:
 // 0 one thread per 5-D site, 1 one thread per 4-D column, 2 one thread per 5-D
 // site with warp-shuffled x neighbours (Nx a multiple of 32), 3 one thread per
 // (s, x) sweeping a chunk of rows in t (Nx a multiple of 32, Ls <= 16), 4 (Wilson
 // only) one thread per kWilsonRows rows of one column from registers, 5 one
-// thread per 4-D column with warp-shuffled x neighbours (Nx a multiple of 32); the
+// thread per 4-D column with warp-shuffled x neighbours; the
 // slice-ring kernel (6) is not a candidate (slower than 5 wherever measured). Unless
 // the context fixes the chunk length, the t sweep is timed at its automatic
 // shape and at chunks of 16, 32, 64 and 128 rows with the widest block and
@@ -381,7 +391,7 @@ DslashChoice pick_variant(dwf_ctx* c, int nrhs, const int* conf_d, int conf0, co
     std::vector<DslashChoice> cand;
     for (int v = 0; v < 6; ++v)
     {
-        if (((v == 2 || v == 5) && c->L.Nx % 32 != 0) || (v == 3 && !sweep_ok(c->L)) ||
+        if ((v == 1 && c->L.Nx % 32 != 0) || (v == 2 && c->L.Nx % 32 != 0) || (v == 3 && !sweep_ok(c->L)) ||
             (v == 4 && !wilson_rows_ok(c->L)))
             continue;
         cand.push_back({v, 0, 0});

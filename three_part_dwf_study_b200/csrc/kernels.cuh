@@ -33,6 +33,13 @@ __global__ void dirac_colx_kernel(Lat L, const cplx<R>* __restrict__ in, cplx<R>
                                   long fsz, const cplx<R>* __restrict__ U, long usz,
                                   const int* __restrict__ conf, int conf0);
 
+// Same operator for any Nx, 32 consecutive sites of the flattened (t, x) plane per
+// warp (grid: ceil(V / 128) x nrhs, 128 threads).
+template <bool DAG, typename R>
+__global__ void dirac_colf_kernel(Lat L, const cplx<R>* __restrict__ in, cplx<R>* __restrict__ out,
+                                  long fsz, const cplx<R>* __restrict__ U, long usz,
+                                  const int* __restrict__ conf, int conf0);
+
 // Same operator over a block-shared ring of kRingSlots slices in shared
 // memory, filled by 1-D bulk copies (cp.async.bulk, mbarrier completion): a
 // block of 8 warps covers 32 x by kRingT t rows and sweeps s; warp 0 copies
