@@ -95,6 +95,9 @@ SIGNATURES = {
     "dwf_set_gauge_dev": (_I, [_P, _I, _P]),
     "dwf_apply": (_I, [_P, _I, _I, _P, _P, _I]),
     "dwf_apply_dev": (_I, [_P, _I, _I, _P, _P, _I, _I]),
+    "dwf_apply_on": (_I, [_P, _I, _I, _P, _P, _I, _I, _P]),
+    "dwf_stream_enter": (_I, [_P, _P]),
+    "dwf_stream_leave": (_I, [_P, _P]),
     "dwf_cg": (_I, [_P, _I, _I, _P, _P, _I, _D, _I, _I, C.POINTER(SolveInfo)]),
     "dwf_cg_batch_dev": (_I, [_P, _I, _I, _P, _P, _P, _I, _D, _I, _I, C.POINTER(SolveInfo)]),
     "dwf_cg_batch": (_I, [_P, _I, _I, _P, _P, _P, _I, _D, _I, _I, C.POINTER(SolveInfo)]),

@@ -98,6 +98,10 @@ int grow(dwf_ctx* c, T*& p, size_t n)
 
 }  // namespace
 
+namespace {
+size_t report_bytes(int nrhs) { return size_t(nrhs) * (2 * sizeof(double) + 3 * sizeof(int)); }
+}  // namespace
+
 int ensure_workspace(dwf_ctx* c, int nrhs)
 {
     if (nrhs <= c->ws_rhs)
@@ -111,13 +115,16 @@ int ensure_workspace(dwf_ctx* c, int nrhs)
         (st = grow(c, c->w_p32, f)) || (st = grow(c, c->w_t32, f)) ||
         (st = grow(c, c->w_e32, f)) || (st = grow(c, c->w_src, f)) ||
         (st = grow(c, c->w_conf, size_t(nrhs))) ||
-        (st = grow(c, c->w_active, size_t(nrhs))) || (st = grow(c, c->w_iters, size_t(nrhs))) ||
-        (st = grow(c, c->w_relres, size_t(nrhs))) || (st = grow(c, c->w_status, size_t(nrhs))) ||
-        (st = grow(c, c->w_ru, size_t(nrhs))) || (st = grow(c, c->w_true, size_t(nrhs))))
+        (st = grow(c, c->w_active, size_t(nrhs))) || (st = grow(c, c->w_rep, report_bytes(nrhs))))
     {
         c->ws_rhs = 0;
         return st;
     }
+    c->w_relres = reinterpret_cast<double*>(c->w_rep);
+    c->w_true = c->w_relres + nrhs;
+    c->w_iters = reinterpret_cast<int*>(c->w_true + nrhs);
+    c->w_status = c->w_iters + nrhs;
+    c->w_ru = c->w_status + nrhs;
     c->ws_rhs = nrhs;
     return DWF_OK;
 }
@@ -486,8 +493,9 @@ int apply_dev(dwf_ctx* c, int op, int nrhs, const int* conf_d, int conf0, const 
     return DWF_OK;
 }
 
-int true_residual(dwf_ctx* c, int op, int nrhs, const int* conf_d, const double2* b,
-                  const double2* x, double* out)
+// Queue the FP64 true residuals |b - A x| / |b| into w_true.
+int queue_true_residual(dwf_ctx* c, int op, int nrhs, const int* conf_d, const double2* b,
+                        const double2* x)
 {
     // t = D1 x
     const bool dag1 = (op == DWF_OP_DDDAG);
@@ -511,6 +519,15 @@ int true_residual(dwf_ctx* c, int op, int nrhs, const int* conf_d, const double2
     residual_finish_kernel<<<(nrhs + 7) / 8, 256, 0, c->stream>>>(c->w_part, nrhs, nch, c->w_true);
     CK(cudaGetLastError());
     c->launches += 3;
+    return DWF_OK;
+}
+
+int true_residual(dwf_ctx* c, int op, int nrhs, const int* conf_d, const double2* b,
+                  const double2* x, double* out)
+{
+    const int st = queue_true_residual(c, op, nrhs, conf_d, b, x);
+    if (st)
+        return st;
     CK(cudaMemcpyAsync(out, c->w_true, nrhs * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
     return DWF_OK;
@@ -521,11 +538,46 @@ namespace {
 constexpr int kSolverThreads = 256;
 constexpr int kMaxRhsPerLaunch = 2048;
 
-// One persistent launch over nrhs <= kMaxRhsPerLaunch right-hand sides.
+struct Reports
+{
+    std::vector<int> iters, status, ru;
+    std::vector<double> relres, true_relres;
+};
+
+// Wait for the launch before and read its reports and the true residuals queued
+// after it: one copy (the host vectors are pageable, so each copy would wait), then
+// the error word.
+int read_reports(dwf_ctx* c, int nrhs, Reports& r)
+{
+    std::vector<unsigned char> h(report_bytes(c->ws_rhs));
+    GridBar hb{};
+    CK(cudaMemcpyAsync(h.data(), c->w_rep, h.size(), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaMemcpyAsync(&hb, c->bar, sizeof(GridBar), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    auto doubles = [&](const double* d) {
+        std::vector<double> v(nrhs);
+        std::memcpy(v.data(), h.data() + (reinterpret_cast<const unsigned char*>(d) - c->w_rep), nrhs * sizeof(double));
+        return v;
+    };
+    auto ints = [&](const int* d) {
+        std::vector<int> v(nrhs);
+        std::memcpy(v.data(), h.data() + (reinterpret_cast<const unsigned char*>(d) - c->w_rep), nrhs * sizeof(int));
+        return v;
+    };
+    r = {ints(c->w_iters), ints(c->w_status), ints(c->w_ru), doubles(c->w_relres), doubles(c->w_true)};
+    float ms = 0.f;
+    CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
+    c->solver_ms[0] += ms;
+    c->solver_launches[0] += 1;
+    if (hb.err != 0)
+        return ctx_fail(c, hb.err, hb.err == DWF_TIMEOUT ? "persistent solver: a wait ran out"
+                                                          : "persistent solver: device error");
+    return DWF_OK;
+}
+
+// Queue one persistent launch over nrhs <= kMaxRhsPerLaunch right-hand sides.
 int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, double2* x,
-                  int has_guess, const int* active_d, double rtol, int maxiter, int eigen_rule,
-                  std::vector<int>& iters, std::vector<double>& relres, std::vector<int>& status,
-                  std::vector<int>& ru)
+                  int has_guess, const int* active_d, double rtol, int maxiter, int eigen_rule)
 {
     SolveDesc d{};
     d.L = c->L;
@@ -600,24 +652,6 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
     }
     CK(cudaEventRecord(c->ev1, c->stream));
     c->launches += 1;
-    GridBar hb{};
-    iters.resize(nrhs);
-    relres.resize(nrhs);
-    status.resize(nrhs);
-    ru.resize(nrhs);
-    CK(cudaMemcpyAsync(iters.data(), c->w_iters, nrhs * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(relres.data(), c->w_relres, nrhs * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(status.data(), c->w_status, nrhs * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(ru.data(), c->w_ru, nrhs * sizeof(int), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(&hb, c->bar, sizeof(GridBar), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    float ms = 0.f;
-    CK(cudaEventElapsedTime(&ms, c->ev0, c->ev1));
-    c->solver_ms[0] += ms;
-    c->solver_launches[0] += 1;
-    if (hb.err != 0)
-        return ctx_fail(c, hb.err, hb.err == DWF_TIMEOUT ? "persistent solver: a wait ran out"
-                                                          : "persistent solver: device error");
     return DWF_OK;
 }
 
@@ -649,51 +683,48 @@ int solve_batch(dwf_ctx* c, int op, int nrhs, const int* conf_h, const double2* 
         std::vector<int> conf(n, 0);
         if (conf_h)
             std::copy(conf_h + k0, conf_h + k0 + n, conf.begin());
-        CK(cudaMemcpyAsync(c->w_conf, conf.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+        if (conf_h)
+            CK(cudaMemcpyAsync(c->w_conf, conf.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+        else
+            CK(cudaMemsetAsync(c->w_conf, 0, n * sizeof(int), c->stream));
         const double2* bk = b + k0 * fs;
         double2* xk = x + k0 * fs;
         if (!has_guess)
             CK(cudaMemsetAsync(xk, 0, size_t(n) * fs * sizeof(double2), c->stream));
-        std::vector<int> iters, status, ru;
-        std::vector<double> relres;
+        Reports r;
         const bool mixed = (solver == DWF_SOLVER_MIXED);
-        st = launch_solver(c, mixed, op, n, bk, xk, has_guess, nullptr, rtol, maxiter, eigen_rule,
-                           iters, relres, status, ru);
-        if (st)
+        // the true residuals are queued behind the solve; only a stalled mixed
+        // right-hand side needs them again
+        if ((st = launch_solver(c, mixed, op, n, bk, xk, has_guess, nullptr, rtol, maxiter, eigen_rule)) ||
+            (st = queue_true_residual(c, op, n, c->w_conf, bk, xk)) || (st = read_reports(c, n, r)))
             return st;
         std::vector<int> fallback(n, 0);
         int nfb = 0;
-        if (mixed)
-        {
-            for (int k = 0; k < n; ++k)
-                if (status[k] != DWF_OK)
-                {
-                    fallback[k] = 1;
-                    ++nfb;
-                }
-            if (nfb)
+        for (int k = 0; mixed && k < n; ++k)
+            if (r.status[k] != DWF_OK)
             {
-                // plain FP64 CG from the mixed iterate for every right-hand side that stalled
-                CK(cudaMemcpyAsync(c->w_active, fallback.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
-                std::vector<int> it2, st2, ru2;
-                std::vector<double> rr2;
-                st = launch_solver(c, false, op, n, bk, xk, 1, c->w_active, rtol, maxiter,
-                                   eigen_rule, it2, rr2, st2, ru2);
-                if (st)
-                    return st;
-                for (int k = 0; k < n; ++k)
-                    if (fallback[k])
-                    {
-                        iters[k] += it2[k];
-                        relres[k] = rr2[k];
-                        status[k] = st2[k];
-                    }
+                fallback[k] = 1;
+                ++nfb;
             }
+        if (nfb)
+        {
+            // plain FP64 CG from the mixed iterate for every right-hand side that stalled
+            CK(cudaMemcpyAsync(c->w_active, fallback.data(), n * sizeof(int), cudaMemcpyHostToDevice, c->stream));
+            Reports f;
+            if ((st = launch_solver(c, false, op, n, bk, xk, 1, c->w_active, rtol, maxiter, eigen_rule)) ||
+                (st = queue_true_residual(c, op, n, c->w_conf, bk, xk)) || (st = read_reports(c, n, f)))
+                return st;
+            for (int k = 0; k < n; ++k)
+                if (fallback[k])
+                {
+                    r.iters[k] += f.iters[k];
+                    r.relres[k] = f.relres[k];
+                    r.status[k] = f.status[k];
+                }
+            r.true_relres = f.true_relres;
         }
-        std::vector<double> tr(n);
-        st = true_residual(c, op, n, c->w_conf, bk, xk, tr.data());
-        if (st)
-            return st;
+        const std::vector<int>&iters = r.iters, &status = r.status, &ru = r.ru;
+        const std::vector<double>&relres = r.relres, &tr = r.true_relres;
         for (int k = 0; info && k < n; ++k)
         {
             dwf_solve_info& I = info[k0 + k];
@@ -887,6 +918,8 @@ int dwfb_ctx_init(dwf_ctx* c, int device)
     CK(cudaMemset(c->bar, 0, sizeof(GridBar)));
     CK(cudaEventCreate(&c->ev0));
     CK(cudaEventCreate(&c->ev1));
+    for (cudaEvent_t& ev : c->join_ev)
+        CK(cudaEventCreateWithFlags(&ev, cudaEventDisableTiming));
     return DWF_OK;
 }
 
@@ -931,7 +964,7 @@ int dwf_ctx_destroy(dwf_ctx* c)
     void* bufs[] = {c->h_mom, c->h_force, c->h_part, c->h_scal, c->h_chi, c->h_phi, c->h_eta,
                     c->h_xi, c->theta, c->U64, c->U32, c->w_r, c->w_p, c->w_p2, c->w_p32b, c->w_t, c->w_b, c->w_x,
                     c->w_r32, c->w_p32, c->w_t32, c->w_e32, c->w_src, c->w_part, c->w_conf, c->w_active,
-                    c->w_iters, c->w_relres, c->w_status, c->w_ru, c->w_true, c->bar, c->dslash_err,
+                    c->w_rep, c->bar, c->dslash_err,
                     c->eo_se, c->eo_so, c->eo_bh, c->eo_rhs_o, c->eo_x, c->eo_r, c->eo_t, c->eo_y,
                     c->eo_xn, c->eo_r32, c->eo_p32, c->eo_t32, c->eo_y32, c->eo_e32,
                     c->eo_phase, c->m_red, c->m_loop, c->m_z4};
@@ -946,6 +979,9 @@ int dwf_ctx_destroy(dwf_ctx* c)
     if (c->ev1)
         cudaEventDestroy(c->ev1);
     for (cudaEvent_t ev : c->pipe_ev)
+        if (ev)
+            cudaEventDestroy(ev);
+    for (cudaEvent_t ev : c->join_ev)
         if (ev)
             cudaEventDestroy(ev);
     if (c->copy_stream)
@@ -1089,6 +1125,38 @@ int dwf_apply_dev(dwf_ctx* c, int op, int conf, const void* in, void* out, int n
         return DWF_BAD_ARG;
     CK(cudaSetDevice(c->device));
     return apply_dev(c, op, nrhs, nullptr, conf, in, out, precision);
+}
+
+// Order the context's stream behind the caller's, and the caller's behind it.
+int dwf_stream_enter(dwf_ctx* c, void* stream)
+{
+    if (!c)
+        return DWF_BAD_ARG;
+    CK(cudaEventRecord(c->join_ev[0], static_cast<cudaStream_t>(stream)));
+    CK(cudaStreamWaitEvent(c->stream, c->join_ev[0], 0));
+    return DWF_OK;
+}
+
+int dwf_stream_leave(dwf_ctx* c, void* stream)
+{
+    if (!c)
+        return DWF_BAD_ARG;
+    CK(cudaEventRecord(c->join_ev[1], c->stream));
+    CK(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), c->join_ev[1], 0));
+    return DWF_OK;
+}
+
+int dwf_apply_on(dwf_ctx* c, int op, int conf, const void* in, void* out, int nrhs, int precision, void* stream)
+{
+    if (!c || !in || !out)
+        return DWF_BAD_ARG;
+    CK(cudaSetDevice(c->device));
+    int st = dwf_stream_enter(c, stream);
+    if (st)
+        return st;
+    st = apply_dev(c, op, nrhs, nullptr, conf, in, out, precision);
+    const int s2 = dwf_stream_leave(c, stream);
+    return st ? st : s2;
 }
 
 int dwf_apply(dwf_ctx* c, int op, int conf, const double* in, double* out, int nrhs)

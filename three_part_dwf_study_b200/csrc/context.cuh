@@ -44,6 +44,7 @@ struct dwf_ctx
     std::map<int, DslashChoice> dslash_tuned;
     // CUDA events bracketing each persistent solver launch on `stream`
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    cudaEvent_t join_ev[2] = {};  // ordering against a caller's stream (dwf_stream_enter / _leave)
     // device time of solver launches: full lattice, even-odd (either kernel),
     // even-odd cluster kernel alone
     double solver_ms[3] = {0.0, 0.0, 0.0};
@@ -82,6 +83,9 @@ struct dwf_ctx
     size_t m_z4_cap = 0;
     int* w_conf = nullptr;
     int* w_active = nullptr;
+    // per-right-hand-side reports, parts of one block so that one copy reads them
+    // back: relres, true residual [ws_rhs] doubles, iters, status, ru [ws_rhs] ints
+    unsigned char* w_rep = nullptr;
     int* w_iters = nullptr;
     double* w_relres = nullptr;
     int* w_status = nullptr;

@@ -40,8 +40,9 @@ int ensure_hmc(dwf_ctx* c)
     return DWF_OK;
 }
 
-// Gauge force of configuration slot 0 into h_force; S_g and sum cos P to host.
-int gauge_force(dwf_ctx* c, double* Sg, double* cos_sum)
+// Gauge force of configuration slot 0 into h_force; S_g and sum cos P stay on the
+// device (h_scal[0], [1]) until read_scalars.
+int gauge_force(dwf_ctx* c)
 {
     gauge_force_kernel<<<kRedBlocks, 256, 0, c->stream>>>(c->L.Nt, c->L.Nx, c->beta, c->theta,
                                                           c->h_force, c->h_part);
@@ -49,12 +50,15 @@ int gauge_force(dwf_ctx* c, double* Sg, double* cos_sum)
     finish_sum_kernel<<<1, 64, 0, c->stream>>>(c->h_part + 1, kRedBlocks, 2, c->h_scal + 1);
     CK(cudaGetLastError());
     c->launches += 3;
-    double h[2];
-    CK(cudaMemcpyAsync(h, c->h_scal, 2 * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
+    return DWF_OK;
+}
+
+// h_scal to the host: S_g, sum cos P, S_pf, kinetic, as last computed. One read of a
+// trajectory's sums at each end; a read per leapfrog step cost a copy and a wait each.
+int read_scalars(dwf_ctx* c, double (&h)[4])
+{
+    CK(cudaMemcpyAsync(h, c->h_scal, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
     CK(cudaStreamSynchronize(c->stream));
-    *Sg = h[0];
-    if (cos_sum)
-        *cos_sum = h[1];
     return DWF_OK;
 }
 
@@ -64,12 +68,11 @@ int gauge_force(dwf_ctx* c, double* Sg, double* cos_sum)
 // (pseudofermion.hpp:32-41). Wilson: started from zero and accepted when the
 // FP64 residual is within 20 tol (wilson/include/cg_solver.hpp:53-78).
 int pf_force(dwf_ctx* c, const double2* phi, int has_guess, double rtol, int maxiter, int solver,
-             double* Spf, dwf_solve_info* info_out)
+             dwf_solve_info* info_out)
 {
     const bool wilson = c->kind == 1;
     dwf_solve_info info{};
-    const int conf0 = 0;
-    int st = solve_batch(c, DWF_OP_DDDAG, 1, &conf0, phi, c->h_eta, wilson ? 0 : has_guess, rtol,
+    int st = solve_batch(c, DWF_OP_DDDAG, 1, nullptr, phi, c->h_eta, wilson ? 0 : has_guess, rtol,
                          maxiter, solver, wilson ? 1 : 0, &info);
     if (st)
         return st;
@@ -99,19 +102,15 @@ int pf_force(dwf_ctx* c, const double2* phi, int has_guess, double rtol, int max
         c->L, c->h_eta, c->h_xi, c->U64, c->h_force);
     CK(cudaGetLastError());
     c->launches += 3;
-    CK(cudaMemcpyAsync(Spf, c->h_scal + 2, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     return DWF_OK;
 }
 
-int kinetic(dwf_ctx* c, double* K)
+int kinetic(dwf_ctx* c)
 {
     kinetic_kernel<<<kRedBlocks, 256, 0, c->stream>>>(c->h_mom, c->usz(), c->h_part);
     finish_sum_kernel<<<1, 64, 0, c->stream>>>(c->h_part, kRedBlocks, 1, c->h_scal + 3);
     CK(cudaGetLastError());
     c->launches += 2;
-    CK(cudaMemcpyAsync(K, c->h_scal + 3, sizeof(double), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
     return DWF_OK;
 }
 
@@ -161,12 +160,11 @@ int dwf_gauge_action_force(dwf_ctx* c, const double* theta, double* action, doub
     int st = begin(c, theta);
     if (st)
         return st;
-    double sg = 0.0;
-    st = gauge_force(c, &sg, nullptr);
-    if (st)
+    double h[4];
+    if ((st = gauge_force(c)) || (st = read_scalars(c, h)))
         return st;
     if (action)
-        *action = sg;
+        *action = h[0];
     if (force)
     {
         CK(cudaMemcpyAsync(force, c->h_force, c->usz() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
@@ -180,11 +178,10 @@ int dwf_average_plaquette(dwf_ctx* c, const double* theta, double* plaquette)
     int st = begin(c, theta);
     if (st)
         return st;
-    double sg = 0.0, cs = 0.0;
-    st = gauge_force(c, &sg, &cs);
-    if (st)
+    double h[4];
+    if ((st = gauge_force(c)) || (st = read_scalars(c, h)))
         return st;
-    *plaquette = cs / double(c->L.V);
+    *plaquette = h[1] / double(c->L.V);
     return DWF_OK;
 }
 
@@ -202,12 +199,12 @@ int dwf_pf_action_force(dwf_ctx* c, const double* theta, const double* phi, cons
     if (eta_guess)
         CK(cudaMemcpyAsync(c->h_eta, eta_guess, fb, cudaMemcpyHostToDevice, c->stream));
     CK(cudaMemsetAsync(c->h_force, 0, c->usz() * sizeof(double), c->stream));
-    double spf = 0.0;
-    st = pf_force(c, c->h_phi, eta_guess != nullptr, rtol, maxiter, solver, &spf, info);
-    if (st)
+    double h[4];
+    if ((st = pf_force(c, c->h_phi, eta_guess != nullptr, rtol, maxiter, solver, info)) ||
+        (st = read_scalars(c, h)))
         return st;
     if (action)
-        *action = spf;
+        *action = h[2];
     if (force)
         CK(cudaMemcpyAsync(force, c->h_force, c->usz() * sizeof(double), cudaMemcpyDeviceToHost, c->stream));
     if (eta_out)
@@ -237,27 +234,27 @@ int dwf_hmc_trajectory(dwf_ctx* c, const dwf_hmc_params* hp, const double* theta
     if ((st = apply_dev(c, DWF_OP_D, 1, nullptr, 0, c->h_chi, c->h_phi, 64)))
         return st;
     dwf_traj_info I{};
-    double sg = 0.0, spf = 0.0, k0 = 0.0;
+    double h[4];
     dwf_solve_info si{};
-    if ((st = gauge_force(c, &sg, nullptr)))
+    if ((st = gauge_force(c)))
         return st;
-    if ((st = pf_force(c, c->h_phi, 0, hp->rtol, hp->maxiter, hp->solver, &spf, &si)))
+    if ((st = pf_force(c, c->h_phi, 0, hp->rtol, hp->maxiter, hp->solver, &si)))
         return st;
     I.cg_iterations += si.iterations;
     I.solves += 1;
-    if ((st = kinetic(c, &k0)))
+    if ((st = kinetic(c)) || (st = read_scalars(c, h)))
         return st;
-    I.kinetic0 = k0;
-    I.H0 = k0 + sg + spf;
+    I.kinetic0 = h[3];
+    I.H0 = h[3] + h[0] + h[2];
     if ((st = kick(c, 0.5 * hp->epsilon)))
         return st;
     for (int step = 0; step < hp->steps; ++step)
     {
         if ((st = drift(c, hp->epsilon, 0)))
             return st;
-        if ((st = gauge_force(c, &sg, nullptr)))
+        if ((st = gauge_force(c)))
             return st;
-        if ((st = pf_force(c, c->h_phi, 1, hp->rtol, hp->maxiter, hp->solver, &spf, &si)))
+        if ((st = pf_force(c, c->h_phi, 1, hp->rtol, hp->maxiter, hp->solver, &si)))
             return st;
         I.cg_iterations += si.iterations;
         I.solves += 1;
@@ -266,18 +263,16 @@ int dwf_hmc_trajectory(dwf_ctx* c, const dwf_hmc_params* hp, const double* theta
     }
     if ((st = kick(c, 0.5 * hp->epsilon)))
         return st;
-    double k1 = 0.0;
-    if ((st = kinetic(c, &k1)))
+    if ((st = kinetic(c)) || (st = read_scalars(c, h)))
         return st;
-    I.kinetic = k1;
-    I.S_gauge = sg;
-    I.S_pf = spf;
-    I.H = k1 + sg + spf;
+    I.kinetic = h[3];
+    I.S_gauge = h[0];
+    I.S_pf = h[2];
+    I.H = h[3] + h[0] + h[2];
     I.dH = I.H - I.H0;
-    double tmp = 0.0, cs = 0.0;
-    if ((st = gauge_force(c, &tmp, &cs)))
+    if ((st = gauge_force(c)) || (st = read_scalars(c, h)))
         return st;
-    I.plaquette = cs / double(c->L.V);
+    I.plaquette = h[1] / double(c->L.V);
     I.acceptance_probability = std::min(std::exp(-I.dH), 1.0);
     I.status = DWF_OK;
     CK(cudaMemcpyAsync(theta_out, c->theta, gb, cudaMemcpyDeviceToHost, c->stream));
@@ -403,26 +398,26 @@ int wil_hmc_step(dwf_ctx* c, const dwf_hmc_params* hp, const double* theta_old,
         return st;
     dwf_traj_info I{};
     dwf_solve_info si{};
-    double sg = 0.0, spf = 0.0, k0 = 0.0;
-    if ((st = gauge_force(c, &sg, nullptr)))
+    double h[4];
+    if ((st = gauge_force(c)))
         return st;
-    if ((st = pf_force(c, c->h_phi, 0, hp->rtol, hp->maxiter, hp->solver, &spf, &si)))
+    if ((st = pf_force(c, c->h_phi, 0, hp->rtol, hp->maxiter, hp->solver, &si)))
         return st;
     I.cg_iterations += si.iterations;
     I.solves += 1;
-    if ((st = kinetic(c, &k0)))
+    if ((st = kinetic(c)) || (st = read_scalars(c, h)))
         return st;
-    I.kinetic0 = k0;
-    I.H0 = k0 + sg + spf;
+    I.kinetic0 = h[3];
+    I.H0 = h[3] + h[0] + h[2];
     if ((st = kick(c, 0.5 * hp->epsilon)))
         return st;
     for (int step = 0; step < hp->steps; ++step)
     {
         if ((st = drift(c, hp->epsilon, 1)))
             return st;
-        if ((st = gauge_force(c, &sg, nullptr)))
+        if ((st = gauge_force(c)))
             return st;
-        if ((st = pf_force(c, c->h_phi, 0, hp->rtol, hp->maxiter, hp->solver, &spf, &si)))
+        if ((st = pf_force(c, c->h_phi, 0, hp->rtol, hp->maxiter, hp->solver, &si)))
             return st;
         I.cg_iterations += si.iterations;
         I.solves += 1;
@@ -430,13 +425,12 @@ int wil_hmc_step(dwf_ctx* c, const dwf_hmc_params* hp, const double* theta_old,
         if ((st = kick(c, factor * hp->epsilon)))
             return st;
     }
-    double k1 = 0.0;
-    if ((st = kinetic(c, &k1)))
+    if ((st = kinetic(c)) || (st = read_scalars(c, h)))
         return st;
-    I.kinetic = k1;
-    I.S_gauge = sg;
-    I.S_pf = spf;
-    I.H = k1 + sg + spf;
+    I.kinetic = h[3];
+    I.S_gauge = h[0];
+    I.S_pf = h[2];
+    I.H = h[3] + h[0] + h[2];
     I.dH = I.H - I.H0;
     I.acceptance_probability = std::min(1.0, std::exp(-I.dH));
     I.accepted = (u < I.acceptance_probability) ? 1 : 0;
@@ -451,10 +445,10 @@ int wil_hmc_step(dwf_ctx* c, const dwf_hmc_params* hp, const double* theta_old,
         if ((st = set_gauge(c, 1, theta_old, cudaMemcpyHostToDevice)))
             return st;
     }
-    double tmp = 0.0, cs = 0.0;  // plaquette of the configuration returned
-    if ((st = gauge_force(c, &tmp, &cs)))
+    // plaquette of the configuration returned
+    if ((st = gauge_force(c)) || (st = read_scalars(c, h)))
         return st;
-    I.plaquette = cs / double(c->L.V);
+    I.plaquette = h[1] / double(c->L.V);
     I.status = DWF_OK;
     if (info)
         *info = I;

@@ -32,6 +32,38 @@ def _ptr(a):
     return C.c_void_p(a.ctypes.data)
 
 
+class _Ordered:
+    """Stream ordering around a device call: by the library where torch's current
+    stream is on the context's device (two native calls), else by torch events."""
+
+    def __init__(self, ctx):
+        import torch
+        self.ctx, self.cur = ctx, torch.cuda.current_stream()
+        self.near = self.cur.device_index == ctx.device
+
+    def __enter__(self):
+        if self.near:
+            self.ctx._check(A.lib().dwf_stream_enter(self.ctx._h, self.cur.cuda_stream))
+            return
+        import torch
+        self.ext = torch.cuda.ExternalStream(self.ctx.stream_ptr())
+        e = torch.cuda.Event()
+        e.record(self.cur)
+        self.ext.wait_event(e)
+
+    def __exit__(self, kind, value, trace):
+        if self.near:
+            st = A.lib().dwf_stream_leave(self.ctx._h, self.cur.cuda_stream)
+            if kind is None:
+                self.ctx._check(st)
+            return False
+        import torch
+        e = torch.cuda.Event()
+        e.record(self.ext)
+        self.cur.wait_event(e)
+        return False
+
+
 class DomainWall(LearnedMixin):
     """One device context for a domain-wall lattice (dwf.Nt, dwf.Nx, dwf.N5,
     dwf.M5, dwf.mf, dwf.beta)."""
@@ -135,23 +167,7 @@ class DomainWall(LearnedMixin):
         queued on torch's current stream (the tensors' producers), and torch's
         current stream waits for the library's work before anything reads the
         results."""
-        import contextlib
-        import torch
-
-        @contextlib.contextmanager
-        def cm():
-            cur = torch.cuda.current_stream()
-            ext = torch.cuda.ExternalStream(self.stream_ptr())
-            e0 = torch.cuda.Event()
-            e0.record(cur)
-            ext.wait_event(e0)
-            try:
-                yield
-            finally:
-                e1 = torch.cuda.Event()
-                e1.record(ext)
-                cur.wait_event(e1)
-        return cm()
+        return _Ordered(self)
 
     def _dev_fields(self, t, what):
         """(precision, nrhs) of a contiguous CUDA tensor holding whole fields.
@@ -184,10 +200,16 @@ class DomainWall(LearnedMixin):
         self._theta = None
 
     def apply_dev(self, op, inp, out, conf=0):
+        import torch
         prec, nrhs = self._dev_fields(inp, "in")
         prec2, nrhs2 = self._dev_fields(out, "out")
         if (prec, nrhs) != (prec2, nrhs2):
             raise ValueError("in/out: precision or field count differ")
+        cur = torch.cuda.current_stream()
+        if cur.device_index == self.device:
+            self._check(A.lib().dwf_apply_on(self._h, op, conf, inp.data_ptr(), out.data_ptr(),
+                                             nrhs, prec, cur.cuda_stream))
+            return
         with self._ordered():
             self._check(A.lib().dwf_apply_dev(self._h, op, conf, C.c_void_p(inp.data_ptr()),
                                               C.c_void_p(out.data_ptr()), nrhs, prec))
