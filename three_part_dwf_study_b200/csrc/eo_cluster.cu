@@ -39,8 +39,13 @@
 // on the same banks four ways, a cluster barrier per phase and remote gathers for
 // the sums; 20.6 with p, r, e in registers; 17.6 with asynchronous stores instead of
 // cluster barriers; 16.2 with sums per CTA and no timer read in the waits (a read of
-// the global timer takes about a message's time); 15.4 with fewer reliable updates.
-// 64x96x16 with 56, which the grid-wide kernel had to take: 113 ms, now 45.
+// the global timer takes about a message's time); 15.1 with fewer reliable updates and
+// no square roots in the stopping test; 14.4 with y and t at the thread's own places
+// kept in registers between the phases (EREG: a quarter of the hops' loads). ncu (256
+// threads, 60 iterations): 3.3 k instructions per warp and iteration, issue 35 % of its
+// peak and shared-memory wavefronts 47 % before that last step, stalls split
+// between shared-memory latency and the exchanges' waits.
+// 64x96x16 with 56, which the grid-wide kernel had to take: 113 ms, now 43.
 //
 // M5^-1 (per spin an Ls x Ls bidiagonal matrix with the m_f corner, closed form
 // in eo.cuh): the two fifth-dimension recurrences run over the thread's slices in
@@ -167,28 +172,31 @@ __device__ __forceinline__ void cl_m5inv(Spinor<R> (&z)[LT], int q, const M5w<R>
     }
 }
 
-// Where the four hop neighbours of a thread's 4-D site sit in a shared field of
-// the other parity (slice 0; every slice is SS further), halo rows included.
+// Where the hop neighbours of a thread's 4-D site sit in a shared field of the other
+// parity (slice 0; every slice is SS further), halo rows included: t +- 1, and of the
+// two x neighbours the one that is not the thread's own place (t, k). The other one
+// is, so the thread that owns both sites has it in registers.
 struct ClNbr
 {
-    int tp, tm, xp, xm;
+    int tp, tm, oth;
 };
 
-__device__ __forceinline__ ClNbr cl_nbr(int Nx, int Nxh, int tl, int x)
+// sg = +1 where the own place is the x + 1 neighbour, -1 where it is x - 1.
+__device__ __forceinline__ ClNbr cl_nbr(int Nxh, int tl, int k, float sg)
 {
-    const int xp = (x + 1 == Nx) ? 0 : x + 1, xm = (x == 0) ? Nx - 1 : x - 1;
-    return {(tl + 2) * Nxh + (x >> 1), tl * Nxh + (x >> 1), (tl + 1) * Nxh + (xp >> 1),
-            (tl + 1) * Nxh + (xm >> 1)};
+    const int row = (tl + 1) * Nxh;
+    return {row + Nxh + k, row - Nxh + k, row + (sg > 0.f ? (k == 0 ? Nxh - 1 : k - 1) : (k + 1 == Nxh ? 0 : k + 1))};
 }
 
 // The four link phases of the hops from (t, x), FP32, boundary signs folded in
-// (exact: the signs are +-1).
+// (exact: the signs are +-1): t + 1, t - 1, then the own and the other x neighbour
+// with the backward one conjugated.
 struct ClLinks
 {
-    float2 t, tm, x, xm;
+    float2 t, tm, own, oth;
 };
 
-__device__ __forceinline__ ClLinks cl_links(const float2* __restrict__ U, const Lat& L, int t, int x)
+__device__ __forceinline__ ClLinks cl_links(const float2* __restrict__ U, const Lat& L, int t, int x, float sg)
 {
     const int Nt = L.Nt, Nx = L.Nx;
     const int tm = (t == 0) ? Nt - 1 : t - 1;
@@ -197,16 +205,38 @@ __device__ __forceinline__ ClLinks cl_links(const float2* __restrict__ U, const 
     const float stm = (t == 0) ? float(L.bct) : 1.f;
     const float sxp = (x == Nx - 1) ? float(L.bcx) : 1.f;
     const float sxm = (x == 0) ? float(L.bcx) : 1.f;
-    return {stp * U[t * Nx + x], stm * U[tm * Nx + x], sxp * U[L.V + t * Nx + x], sxm * U[L.V + t * Nx + xm]};
+    const float2 fw = sxp * U[L.V + t * Nx + x], b = U[L.V + t * Nx + xm];
+    const float2 bw = make_float2(sxm * b.x, -sxm * b.y);
+    return {stp * U[t * Nx + x], stm * U[tm * Nx + x], sg > 0.f ? fw : bw, sg > 0.f ? bw : fw};
 }
 
-// The hop sum of one slice (times -1/2: H) from a shared field at slice offset so.
-template <bool DAG>
-__device__ __forceinline__ Spinor<float> cl_hop(const float4* f, const ClNbr& n, const ClLinks& u, int so)
+// Adds the x hop from the neighbour v on side sk (+1 forward, times k) with link u: the
+// projected half-spinor and its two rows as in hop4, the side a multiplier so that
+// forward and backward need no selection.
+__device__ __forceinline__ void cl_xhop(const Spinor<float>& v, float2 u, float sk, float2& up, float2& lo)
 {
-    float2 up, lo;
-    hop4<DAG, float>(f4s(f[n.tp + so]), f4s(f[n.tm + so]), f4s(f[n.xp + so]), f4s(f[n.xm + so]), u.t, u.tm,
-                     u.x, u.xm, 1.f, 1.f, 1.f, 1.f, up, lo);
+    const float2 h = make_float2(v.s0.x + sk * v.s1.y, v.s0.y - sk * v.s1.x);
+    const float2 w = cmul(u, h);
+    up += w;
+    lo.x -= sk * w.y;
+    lo.y += sk * w.x;
+}
+
+// The hop sum of one slice (times -1/2: H) from a shared field at slice offset so; vo
+// is the own place's spinor, sg its side.
+template <bool DAG>
+__device__ __forceinline__ Spinor<float> cl_hop(const float4* f, const ClNbr& n, const ClLinks& u, float sg, int so,
+                                                const Spinor<float>& vo)
+{
+    constexpr float k = DAG ? 1.f : -1.f;
+    const Spinor<float> a = f4s(f[n.tp + so]), b = f4s(f[n.tm + so]), c = f4s(f[n.oth + so]);
+    float2 w = cmul(u.t, a.s0 + k * a.s1);
+    float2 up = w, lo = k * w;
+    w = cmulc(u.tm, b.s0 - k * b.s1);
+    up += w;
+    lo += -k * w;
+    cl_xhop(vo, u.own, k * sg, up, lo);
+    cl_xhop(c, u.oth, -k * sg, up, lo);
     return {up, lo};
 }
 
@@ -406,7 +436,8 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
     const int q = pl.q, tl = pl.tl, k = pl.k, t = pl.t;
     const bool on = pl.on;
     const int hs = pl.h;
-    const ClNbr en = cl_nbr(c.Nx, Nxh, tl, pl.xe), od = cl_nbr(c.Nx, Nxh, tl, pl.xo);
+    const float sge = (t & 1) ? -1.f : 1.f, sgo = -sge;  // the own place's side, even and odd site
+    const ClNbr en = cl_nbr(Nxh, tl, k, sge), od = cl_nbr(Nxh, tl, k, sgo);
     const int own = (tl + 1) * Nxh + k;
     const int s0 = q * LT;
     // halo rows: a first row is the previous CTA's row after its last, a last
@@ -507,12 +538,13 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
         // back by its lanes in each phase (16 registers otherwise)
         if (on && q < 2)
         {
-            const ClLinks u = cl_links(d.U32 + long(d.rhs_conf[jr]) * d.usz, L, t, q == 0 ? pl.xe : pl.xo);
+            const ClLinks u = cl_links(d.U32 + long(d.rhs_conf[jr]) * d.usz, L, t, q == 0 ? pl.xe : pl.xo,
+                                       q == 0 ? sge : sgo);
             float2* const o = LK + q * 4 * nsite + hs;
             o[0] = u.t;
             o[nsite] = u.tm;
-            o[2 * nsite] = u.x;
-            o[3 * nsite] = u.xm;
+            o[2 * nsite] = u.own;
+            o[3 * nsite] = u.oth;
         }
         __syncwarp();
         // ---- x = 0: r = b (FP32 copy in global memory, field A p = 0); |b|^2 ----
@@ -558,6 +590,9 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
             {
                 ++it;
                 // P5 of the iteration before: p = r + beta p
+                // (EREG) y and t at the own places, kept from the phase that forms them
+                // for the phases that read them: a quarter of the hops' loads
+                Spinor<float> yk[EREG ? LT : 1], tk[EREG ? LT : 1];
                 const float beta = float(cf);
 #pragma unroll
                 for (int j = 0; j < LT; ++j)
@@ -580,12 +615,16 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                         for (int j = 0; j < LT; ++j)
                             if (!PAD || s0 + j < Ls)
                             {
-                                const Spinor<float> v = cl_hop<false>(FA, en, u, (s0 + j) * ss);
+                                const Spinor<float> v = cl_hop<false>(FA, en, u, sge, (s0 + j) * ss, p[j]);
                                 z[j] = {zs * v.s0, zs * v.s1};
                                 fence();
                             }
                     cl_m5inv<false, PAD, NL, float, LT>(z, q, w32);
                     store(fB, z);
+                    if (EREG)
+#pragma unroll
+                        for (int j = 0; j < LT; ++j)
+                            yk[EREG ? j : 0] = z[j];
                 }
                 __syncthreads();
                 clk.mark(0);
@@ -602,12 +641,18 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                         for (int j = 0; j < LT; ++j)
                             if (!PAD || s0 + j < Ls)
                             {
-                                const Spinor<float> v = cl_hop<false>(FA, od, u, fB + (s0 + j) * ss);
+                                const Spinor<float> v = cl_hop<false>(
+                                    FA, od, u, sgo, fB + (s0 + j) * ss,
+                                    EREG ? yk[EREG ? j : 0] : f4s(FA[fB + (s0 + j) * ss + own]));
                                 m[j] = persist::axpy(0.5f, v, m[j]);
                                 a0 += spinor_norm2(m[j]);
                                 fence();
                             }
                     store(0, m);
+                    if (EREG)
+#pragma unroll
+                        for (int j = 0; j < LT; ++j)
+                            tk[EREG ? j : 0] = m[j];
                 }
                 sum.part(1, a0);
                 __syncthreads();
@@ -628,12 +673,18 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                         for (int j = 0; j < LT; ++j)
                             if (!PAD || s0 + j < Ls)
                             {
-                                const Spinor<float> v = cl_hop<true>(FA, en, u, (s0 + j) * ss);
+                                const Spinor<float> v = cl_hop<true>(
+                                    FA, en, u, sge, (s0 + j) * ss,
+                                    EREG ? tk[EREG ? j : 0] : f4s(FA[(s0 + j) * ss + own]));
                                 z[j] = {zs * v.s0, zs * v.s1};
                                 fence();
                             }
                     cl_m5inv<true, PAD, NL, float, LT>(z, q, w32);
                     store(fB, z);
+                    if (EREG)
+#pragma unroll
+                        for (int j = 0; j < LT; ++j)
+                            yk[EREG ? j : 0] = z[j];
                 }
                 __syncthreads();
                 clk.mark(3);
@@ -654,14 +705,16 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     Spinor<float> tv[LT], m[LT];
 #pragma unroll
                     for (int j = 0; j < LT; ++j)
-                        tv[j] = act(j) ? f4s(FA[(s0 + j) * ss + own]) : zero;
+                        tv[j] = EREG ? tk[EREG ? j : 0] : act(j) ? f4s(FA[(s0 + j) * ss + own]) : zero;
                     cl::m5<true, PAD, NL>(tv, m, q, Ls, dg, mf);
                     if (on)
 #pragma unroll
                         for (int j = 0; j < LT; ++j)
                             if (!PAD || s0 + j < Ls)
                             {
-                                const Spinor<float> v = cl_hop<true>(FA, od, u, fB + (s0 + j) * ss);
+                                const Spinor<float> v = cl_hop<true>(
+                                    FA, od, u, sgo, fB + (s0 + j) * ss,
+                                    EREG ? yk[EREG ? j : 0] : f4s(FA[fB + (s0 + j) * ss + own]));
                                 const Spinor<float> ap = persist::axpy(0.5f, v, m[j]);
                                 if (!EREG)
                                     eslot(j) = s2f4(persist::axpy(al, p[j], f4s(eslot(j))));
