@@ -378,8 +378,8 @@ int dwf_barrier_selftest(dwf_ctx* ctx, int missing_blocks, uint64_t limit_ns);
  * than 5 at the sizes measured; a copy wait that runs past the context's
  * timeout leaves the output incomplete and DWF_TIMEOUT in the device error
  * word that the next solve reports), -1 = autotune (default): the first
- * application per (precision, batch-size bucket) times variants 0-5 with
- * CUDA events and keeps the fastest, variant 3 at its automatic shape and at
+ * application per (precision, batch-size bucket) times variants 0-5 (1 only
+ * where Nx is a multiple of 32) with CUDA events and keeps the fastest, variant 3 at its automatic shape and at
  * chunks of 16, 32, 64 and 128 rows with the widest, a half- and a
  * quarter-width block (unless dwf_set_dslash_chunk fixes the chunk). dwf_dslash_variant reports the choice in force for a
  * precision and batch size (-1 if not tuned yet). */
@@ -401,8 +401,9 @@ int dwf_set_dslash_chunk(dwf_ctx* ctx, int rows);
  * DWF_B200_EO_KERNEL=grid makes 0 the default of every context. */
 int dwf_set_eo_kernel(dwf_ctx* ctx, int kernel);
 
-/* Per-phase device timers of the even-odd solver kernel (block 0's view, each
- * phase including the grid barrier that ends it): enable (1) allocates and
+/* Per-phase device timers of the even-odd solver kernel (grid-wide kernel: block 0's
+ * view, each phase including the grid barrier that ends it; cluster kernel: the
+ * right-hand side that took longest): enable (1) allocates and
  * zeroes them, 0 frees them (off by default: no cost). dwf_eo_phase_times
  * returns accumulated ms and counts for the phases 0 hop + M5^-1, 1 M5 - H
  * (|t|^2), 2 alpha reduction, 3 adjoint hop + M5^-1, 4 adjoint combine and

@@ -1084,8 +1084,10 @@ int propagators_pipelined(dwf_ctx* c, int nrhs, const int* rhs_conf, const doubl
         ce = cudaStreamWaitEvent(c->stream, c->pipe_ev[k], 0);
         if (ce != cudaSuccess)
             break;
+        c->eo_shape_rhs = nrhs;
         st = propagators(c, n, rhs_conf ? rhs_conf + k0 : nullptr, c->w_src + k0 * fs, c->w_x + k0 * fs,
                          rtol, maxiter, solver, info ? info + k0 : nullptr);
+        c->eo_shape_rhs = 0;
         if (st)
             break;
         ce = cudaEventRecord(c->pipe_ev[4 + k], c->stream);

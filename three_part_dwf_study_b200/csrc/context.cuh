@@ -109,6 +109,9 @@ struct dwf_ctx
     float2* eo_t32 = nullptr;
     float2* eo_y32 = nullptr;
     float2* eo_e32 = nullptr;
+    // right-hand sides the even-odd cluster shape is chosen for (0: the launch's own),
+    // so that the chunks of one batch are solved as the whole batch would be
+    int eo_shape_rhs = 0;
     unsigned long long* eo_phase = nullptr;  // per-phase timers (dwf_eo_phase_profile)
     int eo_kernel = -1;  // even-odd solver kernel: -1 automatic, 0 grid-wide (dwf_set_eo_kernel)
     // captured even-odd propagator chunks (source preparation, the cluster

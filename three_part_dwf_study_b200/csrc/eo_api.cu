@@ -251,7 +251,8 @@ int propagators_eo(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, 
                 uintptr_t(c->eo_p32), uintptr_t(c->eo_t32), uintptr_t(c->eo_y32), uintptr_t(c->eo_e32),
                 uintptr_t(c->w_iters), uintptr_t(c->w_relres), uintptr_t(c->w_status), uintptr_t(c->w_ru),
                 uintptr_t(c->eo_phase), uintptr_t(c->bar), uintptr_t(maxiter), uintptr_t(c->timeout_ns),
-                uintptr_t(std::llround(std::log2(tol) * 1e6)), uintptr_t(d.ru_period)};
+                uintptr_t(std::llround(std::log2(tol) * 1e6)), uintptr_t(d.ru_period),
+                uintptr_t(c->eo_shape_rhs)};
             st = run_graph(c, key, [&]() -> int {
                 int s2 = prepare();
                 if (s2)

@@ -948,7 +948,7 @@ int launch_eo_cluster(dwf_ctx* c, EoDesc& e, bool* launched, bool dry, int* wave
 {
     *launched = false;
     const Lat& L = c->L;
-    const ClShape sh = cl_shape(c, std::max(1, e.d.nrhs));
+    const ClShape sh = cl_shape(c, std::max(1, c->eo_shape_rhs > 0 ? c->eo_shape_rhs : e.d.nrhs));
     if (!sh.fn)
         return DWF_BAD_ARG;
     if (dry)
