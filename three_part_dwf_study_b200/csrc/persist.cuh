@@ -198,16 +198,6 @@ struct DirLd
     __device__ __forceinline__ cplx<R> c(long idx) const { return r[idx] + beta * p[idx]; }
 };
 
-template <typename R, typename Ld>
-__device__ __forceinline__ Spinor<R> op_site_ld(const SolveDesc& d, bool dag, const Ld& in,
-                                                const cplx<R>* __restrict__ U, int i)
-{
-    int s, t, x;
-    site_coords(d.L, i, s, t, x);
-    return dag ? dirac_site_ld<true, R>(in, U, d.L, s, t, x)
-               : dirac_site_ld<false, R>(in, U, d.L, s, t, x);
-}
-
 __device__ inline void write_outputs(const SolveDesc& d, const Smem& s)
 {
     if (blockIdx.x != 0)
