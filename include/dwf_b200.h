@@ -361,6 +361,16 @@ int dwf_cg_noalloc(const dwf_params* params, int op, const double* theta_dev, co
  * into limit_ns and returns DWF_TIMEOUT with the context still usable. */
 int dwf_barrier_selftest(dwf_ctx* ctx, int missing_blocks, uint64_t limit_ns);
 
+/* Self test of the waits inside the solvers that exchange partial sums without the
+ * grid barrier: in each solve from now on one block waits for a sum that no block
+ * sends, so that the wait runs into the limit (dwf_set_wait_limit), the solve returns
+ * DWF_TIMEOUT and the context stays usable. 0 (default): none. Cluster kernels: bit 0
+ * |r|^2 and bit 1 <p, A p> of an iteration, bit 2 |b|^2 (even-odd: and the FP64
+ * residual of a reliable update), bit 3 (full lattice) the starting and the FP64
+ * residual. The whole-GPU kernel of one right-hand side: any bit, from its third sum
+ * on. The kernels with a grid barrier ignore it. */
+int dwf_set_missing_sums(dwf_ctx* ctx, unsigned sums);
+
 /* Dslash kernel variant for dwf_apply[_dev]: 0 = one thread per 5-D site,
  * 1 = one thread per 4-D site sweeping the fifth dimension (links and fifth-
  * dimension neighbours kept in registers), 2 = one thread per 5-D site with

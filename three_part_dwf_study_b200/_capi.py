@@ -111,6 +111,7 @@ SIGNATURES = {
     "dwf_dslash_variant": (_I, [_P, _I, _I]),
     "dwf_set_dslash_chunk": (_I, [_P, _I]),
     "dwf_barrier_selftest": (_I, [_P, _I, C.c_uint64]),
+    "dwf_set_missing_sums": (_I, [_P, C.c_uint]),
     "dwf_cg_noalloc": (_I, [C.POINTER(DwfParams), _I, _P, _P, _P, _I, _D, _I, _P,
                             C.POINTER(SolveInfo)]),
     "dwf_measure": (_I, [_P, C.POINTER(MeasureParams), _I, _P, _P, _P, _P, _P, _P,

@@ -615,6 +615,7 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
     d.out_ru = c->w_ru;
     d.bar = c->bar;
     d.timeout_ns = c->timeout_ns;
+    d.mute = c->mute;
 
     // lattices that fit a cluster: one cluster per right-hand side; else one
     // right-hand side: the whole-GPU latency kernel, batches: work units
@@ -1347,6 +1348,14 @@ int dwf_barrier_selftest(dwf_ctx* c, int missing_blocks, uint64_t limit_ns)
     CK(cudaStreamSynchronize(c->stream));
     if (hb.err != 0)
         return ctx_fail(c, hb.err, "grid barrier wait ran out");
+    return DWF_OK;
+}
+
+int dwf_set_missing_sums(dwf_ctx* c, unsigned sums)
+{
+    if (!c || sums > 15u)
+        return DWF_BAD_ARG;
+    c->mute = sums;
     return DWF_OK;
 }
 

@@ -36,7 +36,7 @@ namespace cg = cooperative_groups;
 
 constexpr int kThreads = 512;
 constexpr int kSlots = 4;  // sums: |r|^2, |t|^2, |b|^2 and the replaced |r|^2
-constexpr size_t kHead = (cl::sum_bytes(kSlots) + (kSlots + 4) * 8 + 15) / 16 * 16;
+constexpr size_t kHead = (cl::sum_bytes(kSlots) + (kSlots + 6) * 8 + 15) / 16 * 16;
 
 struct CgGeo
 {
@@ -185,6 +185,8 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
     cplx<R>* const LK = reinterpret_cast<cplx<R>*>(base + 2 * fT);  // links [4][sites]
     const int nsite = int(blockDim.x) / NL;
     const cl::Sum sum{tab, tab + kSlots * cl::kMaxCtas, bars, CS, rank};
+    const cl::Meet meet{bars + (kSlots + 4) * 8};
+    const cl::Quit quit{meet.word + 8u};
 
     const CgPlace pl = cg_place<NL>(L, g, rank);
     const int q = pl.q, s0 = q * LT, tl = pl.tl, x = pl.x;
@@ -207,7 +209,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
         return v;
     };
     unsigned par = 0;  // barrier parities: bits 0-3 sums, 4 and 5 the halos of p and t
-    int bad = 0;
+    int bad = 0, it = 0;
     auto store = [&](int f, const Spinor<R> (&v)[LT]) {
         const int ss = stride();
         const SField<R> F = field(f ? fT : 0);
@@ -229,7 +231,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
     };
     auto halo = [&](int f) {
         const unsigned b = hbar + 16u * f, ph = (par >> (kSlots + f)) & 1u;
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0 && !bad)
         {
             cl::bar_expect(b, unsigned(Ls * Nx) * unsigned(2 * sizeof(cplx<R>)));
             cl::bar_expect(b + 8u, unsigned(Ls * Nx) * unsigned(2 * sizeof(cplx<R>)));
@@ -239,27 +241,24 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
         if ((threadIdx.x & 31) == 0)
         {
             if (lo)
-                bad = bad || !cl::bar_wait(b, ph, d.timeout_ns);
+                cl::wait(b, ph, d.timeout_ns, quit, it, bad);
             if (hi)
-                bad = bad || !cl::bar_wait(b + 8u, ph, d.timeout_ns);
+                cl::wait(b + 8u, ph, d.timeout_ns, quit, it, bad);
         }
         __syncwarp();
         par ^= (1u << kSlots) << f;
     };
     auto total = [&](int slot) {
-        double v;
-        bad |= !sum.get(slot, (par >> slot) & 1u, bad ? 0ull : d.timeout_ns, v);
+        const double v = sum.get(slot, (par >> slot) & 1u, d.timeout_ns, quit, it, bad);
         par ^= 1u << slot;
         return v;
     };
-    // part(slot) of every warp, a block barrier, the CTA's sum on its way; whether
-    // any thread's wait ran out before
+    // part(slot) of every warp, a block barrier, the CTA's sum on its way
     auto put = [&](int slot, double v) {
         sum.part(slot, v);
-        const int gave_up = __syncthreads_or(bad);
+        __syncthreads();
         if (threadIdx.x < 32)
             sum.send(slot);
-        return gave_up != 0;
     };
     // D (D^dag when dag) of shared field f at this thread's slices
     auto apply = [&](int f, bool dag, Spinor<R> (&o)[LT]) {
@@ -305,7 +304,9 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
     if (threadIdx.x == 0)
     {
         for (int i = 0; i < kSlots + 4; ++i)
-            cl::bar_init(bars + 8u * i);
+            cl::bar_init(bars + 8u * i, i < kSlots && rank + 1 == CS ? (d.mute >> i) & 1u : 0u);
+        meet.init();
+        asm volatile("st.shared::cta.u32 [%0], 0;" ::"r"(quit.word) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cl::sync();
@@ -362,11 +363,14 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
         put(3, a1);
         double rr = total(3);
         double rru = rr, cf = 0.0;
-        int it = 0, iters = 0, ru = 0, stalls = 0;
+        it = 0;
+        int iters = 0, ru = 0, stalls = 0;
         int state = (bb == 0.0 || persist::converged_now(d, rr, bb)) ? DWF_OK : RHS_ACTIVE;
 
-        // Mixed: one pass between two reliable updates. FP64: one pass.
-        bool gave = false;
+        // Mixed: one pass between two reliable updates. FP64: one pass. `gave` is the
+        // same in all threads of the CTA, and so is every value taken from a sum once
+        // it is false.
+        bool gave = __syncthreads_or(bad) != 0;
         while (state == RHS_ACTIVE && it < d.maxiter && !gave)
         {
             Spinor<R> r[LT], xe[LT];
@@ -387,7 +391,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
                     }
                 }
             }
-            bool want = false;
+            bool want = false, zden = false;
             do
             {
                 ++it;
@@ -402,6 +406,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
                     store(0, p);
                 }
                 __syncthreads();
+                gave = quit.at(it);
                 // t = D1 p, |t|^2
                 halo(0);
                 {
@@ -414,23 +419,18 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
                         if (act(j))
                             a0 += spinor_norm2(o[j]);
                 }
-                if (put(1, a0))
-                {
-                    gave = true;
+                if (gave)
                     break;
-                }
+                put(1, a0);
                 // x += alpha p; r -= alpha D2 t; |r|^2
                 halo(1);
                 Spinor<R> ap[LT];
                 apply(1, !dag1, ap);
                 const double tt = total(1);
-                if (MIXED ? (tt == 0.0 || !isfinite(tt)) : tt == 0.0)
-                {
-                    state = MIXED ? DWF_NOT_CONVERGED : DWF_ZERO_DENOM;  // cg_solver.hpp:45-46
-                    iters = it;
-                    break;
-                }
-                const R al = R(rr / tt);
+                // a zero denominator ends the solve with x as it is (FP64: t = D1 p = 0
+                // has a finite p, so 0 p adds nothing; mixed: e is dropped)
+                zden = MIXED ? (tt == 0.0 || !isfinite(tt)) : tt == 0.0;
+                const R al = zden ? R(0) : R(rr / tt);
                 a0 = 0.0;
                 {
                     const int ss = stride();
@@ -447,21 +447,29 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
                 const double rn = total(0);
                 iters = it;
                 if constexpr (MIXED)
-                    want = rn < d.delta * d.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
+                    want = zden || rn < d.delta * d.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
                 else
                 {
-                    if (persist::converged_now(d, rn, bb))
+                    if (!zden && persist::converged_now(d, rn, bb))
                     {
                         iters = d.eigen_rule ? it - 1 : it;
                         state = DWF_OK;
                     }
-                    want = state == DWF_OK || it == d.maxiter;
+                    want = zden || state == DWF_OK || it == d.maxiter;
                 }
                 cf = rn / rr;
-                rr = rn;
+                rr = zden ? rr : rn;
             } while (!want);
+            // (a warp whose sum ran out may be at the next iteration's first barrier)
+            if (!gave)
+            {
+                __syncthreads();
+                gave = quit.at(it + 1);
+            }
             if (gave)
                 break;
+            if (zden)
+                state = MIXED ? DWF_NOT_CONVERGED : DWF_ZERO_DENOM;  // cg_solver.hpp:45-46
 #pragma unroll
             for (int j = 0; j < LT; ++j)
                 if (act(j))
@@ -479,9 +487,14 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
             if (MIXED && state == RHS_ACTIVE)
             {
                 // reliable update in FP64: x += e, r = b - A x
-                cl::sync_global();
+                if (meet(false, CS))
+                {
+                    cl::settle();
+                    return;
+                }
                 put(3, cg_residual<LT, NL, MIXED>(d, g, rank, jr));
                 const double rt = total(3);
+                gave = __syncthreads_or(bad) != 0;
                 ru += 1;
                 cf = cf * (rt / rr);
                 stalls = (rt >= 0.5 * rru) ? stalls + 1 : 0;
@@ -493,14 +506,9 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
                     state = DWF_NOT_CONVERGED;
             }
         }
-        if (__syncthreads_or(bad))
-        {
-            if (threadIdx.x == 0)
-                raise_error(d.bar, DWF_TIMEOUT);
-            cl::linger(d.timeout_ns);
-            return;
-        }
-        if (rank == 0 && threadIdx.x == 0)
+        if (gave && threadIdx.x == 0)
+            raise_error(d.bar, DWF_TIMEOUT);
+        if (!gave && rank == 0 && threadIdx.x == 0)
         {
             d.out_iters[jr] = iters;
             d.out_status[jr] = state == RHS_ACTIVE ? DWF_NOT_CONVERGED : state;
@@ -508,7 +516,11 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
             d.out_ru[jr] = ru;
         }
         // the next right-hand side overwrites the fields and links
-        cl::sync();
+        if (meet(gave, CS))
+        {
+            cl::settle();
+            return;
+        }
     }
     // no CTA leaves while another may still store into its shared memory
     cl::sync();

@@ -12,6 +12,11 @@
 // A receiver's barrier is used for one message at a time: the sender's next
 // message into the same place needs data the receiver sends only after it has
 // read the last one (each solver says why at its phases).
+//
+// A wait that runs past the limit is noted in the waiting lane (`bad`) and in the CTA's
+// shared memory (Quit). The warps of a CTA may then hold different values of a sum,
+// so nothing that decides which barrier comes next is taken from a sum before all
+// threads know that none has; a CTA that gives up goes to the next check point (Meet).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -58,9 +63,10 @@ __device__ __forceinline__ void send(unsigned a, double2 v, unsigned bar)
                  : "memory");
 }
 
-__device__ __forceinline__ void bar_init(unsigned bar)
+// One arrival a phase; `missing` more that never come let no phase end (self test).
+__device__ __forceinline__ void bar_init(unsigned bar, unsigned missing = 0)
 {
-    asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(bar) : "memory");
+    asm volatile("mbarrier.init.shared::cta.b64 [%0], %1;" ::"r"(bar), "r"(1u + missing) : "memory");
 }
 // The phase's one arrival, with the bytes it waits for (they may have begun to
 // land before).
@@ -105,11 +111,43 @@ __device__ __forceinline__ void sync_global()
     cg::this_cluster().sync();
 }
 
+// The iteration from which a CTA gives up: one more than the iteration in which a
+// wait ran out first (shared memory, zero: none has). All threads read it between the
+// block barrier that starts an iteration and the next one; noted numbers lie beyond the
+// iteration then, so all get the same answer however late they read.
+struct Quit
+{
+    unsigned word;  // shared address
+
+    __device__ __forceinline__ void from(int it) const
+    {
+        unsigned old;
+        asm volatile("atom.shared::cta.cas.b32 %0, [%1], 0, %2;" : "=r"(old) : "r"(word), "r"(it) : "memory");
+    }
+    __device__ __forceinline__ bool at(int it) const
+    {
+        unsigned v;
+        asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(word) : "memory");
+        return v - 1u < unsigned(it);
+    }
+};
+
+// One lane's wait in iteration `it`. A lane that is bad waits no more.
+__device__ __forceinline__ void wait(unsigned bar, unsigned parity, unsigned long long limit_ns, const Quit& quit,
+                                     int it, int& bad)
+{
+    if (!bad && !bar_wait(bar, parity, limit_ns))
+    {
+        bad = 1;
+        quit.from(it + 1);
+    }
+}
+
 // Sum over the cluster of one value per thread, in three steps: part() leaves
 // every warp's sum in shared memory; after a block barrier send() (by one warp)
 // adds them and sends the CTA's sum to every CTA's table; get() waits for the
 // table and adds it up in a fixed order, the same bits in every warp of every
-// CTA. One lane per warp polls: all threads polling, and a message per warp
+// CTA (unless the wait ran out: bad). One lane per warp polls: all threads polling, and a message per warp
 // instead of per CTA, made the mbarrier the bottleneck (2.5 us a sum at 16 CTAs of
 // 16 warps against 0.5). Thread 0 arms the slot's barrier in get(). A slot
 // is sent again only after every warp of every CTA has sent something that it
@@ -134,19 +172,20 @@ struct Sum
         if (lane < CS)
             cl::send(map(smem_addr(tab + slot * kMaxCtas + rank), lane), v, map(bar + 8u * slot, lane));
     }
-    __device__ __forceinline__ bool get(int slot, unsigned parity, unsigned long long limit_ns, double& v) const
+    // Thread 0 arms no more once it is bad (its barrier may still be in the phase it
+    // armed last).
+    __device__ __forceinline__ double get(int slot, unsigned parity, unsigned long long limit_ns, const Quit& quit,
+                                          int it, int& bad) const
     {
         const int lane = threadIdx.x & 31;
-        bool ok = true;
-        if (lane == 0)
+        if (lane == 0 && !bad)
         {
             if (threadIdx.x == 0)
                 bar_expect(bar + 8u * slot, unsigned(CS) * 8u);
-            ok = bar_wait(bar + 8u * slot, parity, limit_ns);
+            wait(bar + 8u * slot, parity, limit_ns, quit, it, bad);
         }
         __syncwarp();
-        v = warp_sum(lane < CS ? tab[slot * kMaxCtas + lane] : 0.0);
-        return ok;
+        return warp_sum(lane < CS ? tab[slot * kMaxCtas + lane] : 0.0);
     }
 };
 __host__ __device__ constexpr size_t sum_bytes(int nslot)
@@ -154,13 +193,50 @@ __host__ __device__ constexpr size_t sum_bytes(int nslot)
     return size_t(nslot) * (kMaxCtas + kMaxWarps) * sizeof(double);
 }
 
-// A CTA that gave up a wait stays until the others of its cluster have given up
-// theirs too (each waits for it within a phase or two), so that none of them
-// stores into the shared memory of a CTA that has left.
-__device__ __forceinline__ void linger(unsigned long long limit_ns)
+// Check points: the cluster barriers at which the CTAs of a cluster agree on whether
+// one of them gave up. Every CTA passes the same check points in the same order, and
+// all leave at the first one that a CTA reached with `gave`, so no CTA stores into the
+// shared memory of one that has left and none waits at a barrier that another will
+// not reach. The barrier ends: a CTA gets there after at most two of its limited waits
+// once another has stopped sending, and cluster barriers other than check points lie
+// only where no CTA can give up since the last check point.
+//
+// A CTA that gives up writes the number of its next check point into every CTA's
+// word; one that has passed its last check point may do so before a slower one
+// has read its own word there, hence the number and not a flag. True: leave.
+//
+// The word and the count of check points passed lie in shared memory (8 bytes at
+// `word`): a register each would cost the solvers' loops spills. Thread 0 counts after
+// the barrier; every solver has a block barrier before its next check point.
+struct Meet
+{
+    unsigned word;  // shared address
+
+    __device__ __forceinline__ void init() const  // by one thread, before the first cluster barrier
+    {
+        asm volatile("st.shared::cta.v2.u32 [%0], {%1, %1};" ::"r"(word), "r"(0) : "memory");
+    }
+    __device__ __forceinline__ bool operator()(bool gave, int CS) const
+    {
+        unsigned n, v;
+        asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(n) : "r"(word + 4u) : "memory");
+        ++n;
+        if (gave && int(threadIdx.x) < CS)
+            asm volatile("st.shared::cluster.u32 [%0], %1;" ::"r"(map(word, int(threadIdx.x))), "r"(n) : "memory");
+        sync_global();
+        asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(word) : "memory");
+        if (threadIdx.x == 0)
+            asm volatile("st.shared::cta.u32 [%0], %1;" ::"r"(word + 4u), "r"(n) : "memory");
+        return v == n;
+    }
+};
+
+// After a check point that says to leave: all messages have been sent, those still on
+// their way land long before this returns (they take about a microsecond).
+__device__ __forceinline__ void settle()
 {
     const unsigned long long t0 = globaltimer_ns();
-    while (globaltimer_ns() - t0 < 3 * limit_ns)
+    for (int i = 0; i < 100000 && globaltimer_ns() - t0 < 1000000ull; ++i)
         __nanosleep(1000);
 }
 

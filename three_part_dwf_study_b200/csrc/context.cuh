@@ -22,6 +22,7 @@ struct dwf_ctx
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t pipe_ev[8] = {};
     uint64_t timeout_ns = 5000000000ull;
+    unsigned mute = 0;  // sums waited for that are never sent (dwf_set_missing_sums)
     std::string err;
     uint64_t gauge_version = 0;  // bumped whenever the links change
     struct LpNet* lp = nullptr;  // learned preconditioner (dwf_lp_init)

@@ -226,6 +226,7 @@ int propagators_eo(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, 
         d.out_ru = c->w_ru;
         d.bar = c->bar;
         d.timeout_ns = c->timeout_ns;
+        d.mute = c->mute;
         e.g = g;
         e.y64 = c->eo_y;
         e.y32 = c->eo_y32;
@@ -252,7 +253,7 @@ int propagators_eo(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, 
                 uintptr_t(c->w_iters), uintptr_t(c->w_relres), uintptr_t(c->w_status), uintptr_t(c->w_ru),
                 uintptr_t(c->eo_phase), uintptr_t(c->bar), uintptr_t(maxiter), uintptr_t(c->timeout_ns),
                 uintptr_t(std::llround(std::log2(tol) * 1e6)), uintptr_t(d.ru_period),
-                uintptr_t(c->eo_shape_rhs)};
+                uintptr_t(c->eo_shape_rhs), uintptr_t(c->mute)};
             st = run_graph(c, key, [&]() -> int {
                 int s2 = prepare();
                 if (s2)

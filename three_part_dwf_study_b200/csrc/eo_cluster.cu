@@ -74,7 +74,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr size_t kClHead = (cl::sum_bytes(3) + 7 * 8 + 15) / 16 * 16;  // sum tables and mbarriers
+constexpr size_t kClHead = (cl::sum_bytes(3) + 9 * 8 + 15) / 16 * 16;  // sum tables, mbarriers, Meet and Quit
 
 struct ClDesc
 {
@@ -431,6 +431,8 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
     float4* const ES = FA + 2 * Ls * SS;                              // !EREG: e, [LT][threads]
     float2* const LK = reinterpret_cast<float2*>(ES + (EREG ? 0 : LT * int(blockDim.x)));  // links [even, odd][4][sites]
     const cl::Sum sum{tab, tab + 3 * cl::kMaxCtas, bars, CS, rank};
+    const cl::Meet meet{bars + 7 * 8};
+    const cl::Quit quit{meet.word + 8u};
     // lane D q + i of warp w (D = 32 / NL): part q of 4-D site D w + i of each parity
     const ClPlace pl = cl_place<NL>(c, rank);
     const int q = pl.q, tl = pl.tl, k = pl.k, t = pl.t;
@@ -477,11 +479,11 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
     };
     // Parities of the barriers: bits 0-2 sums, 3 and 4 the halos of A and B.
     unsigned par = 0;
-    int bad = 0;
+    int bad = 0, it = 0;
     // Wait for the halo rows this thread reads from field A (f = 0) or B.
     auto halo = [&](int f) {
         const unsigned b = hbar + 16u * f, ph = (par >> (3 + f)) & 1u;
-        if (threadIdx.x == 0)
+        if (threadIdx.x == 0 && !bad)
         {
             cl::bar_expect(b, unsigned(Ls * Nxh) * 16u);
             cl::bar_expect(b + 8u, unsigned(Ls * Nxh) * 16u);
@@ -492,23 +494,24 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
         if ((threadIdx.x & 31) == 0)
         {
             if (lo)
-                bad = bad || !cl::bar_wait(b, ph, d.timeout_ns);
+                cl::wait(b, ph, d.timeout_ns, quit, it, bad);
             if (hi)
-                bad = bad || !cl::bar_wait(b + 8u, ph, d.timeout_ns);
+                cl::wait(b + 8u, ph, d.timeout_ns, quit, it, bad);
         }
         __syncwarp();
         par ^= 8u << f;
     };
     auto total = [&](int slot) {
-        double v;
-        bad |= !sum.get(slot, (par >> slot) & 1u, bad ? 0ull : d.timeout_ns, v);
+        const double v = sum.get(slot, (par >> slot) & 1u, d.timeout_ns, quit, it, bad);
         par ^= 1u << slot;
         return v;
     };
     if (threadIdx.x == 0)
     {
         for (int i = 0; i < 7; ++i)
-            cl::bar_init(bars + 8u * i);
+            cl::bar_init(bars + 8u * i, i < 3 && rank + 1 == CS ? (d.mute >> i) & 1u : 0u);
+        meet.init();
+        asm volatile("st.shared::cta.u32 [%0], 0;" ::"r"(quit.word) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cl::sync();
@@ -564,15 +567,18 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
             sum.send(2);
         const double bb = total(2);
         double rr = bb, rru = bb, cf = 0.0;
-        int it = 0, ru = 0, stalls = 0;
+        it = 0;
+        int ru = 0, stalls = 0;
         int state = (bb == 0.0 || persist::converged_now(d, rr, bb) || d.maxiter < 1) ? DWF_OK : RHS_ACTIVE;
         if (state == DWF_OK && !(bb == 0.0 || persist::converged_now(d, rr, bb)))
             state = DWF_NOT_CONVERGED;
 
         clk.start();
         // Between two reliable updates: p and r come from memory (p from field
-        // A's own places), e starts at zero.
-        while (state == RHS_ACTIVE)
+        // A's own places), e starts at zero. `gave` is the same in all threads of the
+        // CTA, and so is every value taken from a sum once it is false.
+        bool gave = __syncthreads_or(bad) != 0;
+        while (state == RHS_ACTIVE && !gave)
         {
             Spinor<float> p[LT], r[LT], ev[EREG ? LT : 1];
 #pragma unroll
@@ -585,7 +591,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 else
                     ev[EREG ? j : 0] = zero;
             }
-            bool want = false;
+            bool want = false, zden = false;
             do
             {
                 ++it;
@@ -598,8 +604,8 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 for (int j = 0; j < LT; ++j)
                     p[j] = persist::axpy(beta, p[j], r[j]);
                 store(0, p);
-                if (__syncthreads_or(bad))
-                    break;
+                __syncthreads();
+                gave = quit.at(it);
                 clk.mark(6);
                 // P1: y = M5^-1 H_eo p
                 halo(0);
@@ -626,6 +632,8 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                         for (int j = 0; j < LT; ++j)
                             yk[EREG ? j : 0] = z[j];
                 }
+                if (gave)
+                    break;
                 __syncthreads();
                 clk.mark(0);
                 // P2: t = M5 p - H_oe y, |t|^2
@@ -689,11 +697,8 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 __syncthreads();
                 clk.mark(3);
                 const double tt = total(1);
-                if (tt == 0.0 || !isfinite(tt))
-                {
-                    state = DWF_NOT_CONVERGED;
-                    break;
-                }
+                // ends the solve after this phase, e and r dropped
+                zden = tt == 0.0 || !isfinite(tt);
                 const float al = float(rr / tt);
                 clk.mark(2);
                 // P4: Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap; |r|^2
@@ -731,16 +736,22 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     sum.send(0);
                 clk.mark(4);
                 const double rn = total(0);
-                want = rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
+                want = zden || rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
                 cf = rn / rr;
-                rr = rn;
+                rr = zden ? rr : rn;
                 clk.mark(5);
             } while (!want);
-            if (__syncthreads_or(bad))
-                break;
-            if (state != RHS_ACTIVE)
+            // (a warp whose sum ran out may be at the next iteration's first barrier)
+            if (!gave)
             {
-                halo(1);  // the y rows on their way
+                __syncthreads();
+                gave = quit.at(it + 1);
+            }
+            if (gave)
+                break;
+            if (zden)
+            {
+                state = DWF_NOT_CONVERGED;
                 break;
             }
             // ---- reliable update in FP64: x += e, r = b - Dhat^dag Dhat x ----
@@ -755,13 +766,18 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     st_spinor(xj, gi, Spinor<double>{xo.s0 + de.s0, xo.s1 + de.s1});
                     FA[(s0 + j) * SS + own] = s2f4(p[j]);
                 }
-            cl::sync_global();
+            if (meet(false, CS))
+            {
+                cl::settle();
+                return;
+            }
             a0 = cl_reliable<LT, NL, PAD>(e, c, rank, jr);
             sum.part(2, a0);
             __syncthreads();
             if (threadIdx.x < 32)
                 sum.send(2);
             const double rt = total(2);
+            gave = __syncthreads_or(bad) != 0;
             ru += 1;
             cf = cf * (rt / rr);
             stalls = (rt >= 0.5 * rru) ? stalls + 1 : 0;
@@ -773,15 +789,10 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 state = DWF_NOT_CONVERGED;
             clk.mark(5);
         }
-        if (__syncthreads_or(bad))
-        {
-            if (threadIdx.x == 0)
-                raise_error(d.bar, DWF_TIMEOUT);
-            cl::linger(d.timeout_ns);
-            return;
-        }
+        if (gave && threadIdx.x == 0)
+            raise_error(d.bar, DWF_TIMEOUT);
         clk.report();
-        if (rank == 0 && threadIdx.x == 0)
+        if (!gave && rank == 0 && threadIdx.x == 0)
         {
             d.out_iters[jr] = it;
             d.out_status[jr] = state;
@@ -789,7 +800,11 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
             d.out_ru[jr] = ru;
         }
         // the next right-hand side overwrites the fields and partials
-        cl::sync();
+        if (meet(gave, CS))
+        {
+            cl::settle();
+            return;
+        }
     }
 }
 

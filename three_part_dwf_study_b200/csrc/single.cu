@@ -140,17 +140,18 @@ struct GridSum
     double* sm;         // [64] shared
     GridBar* bar;
     unsigned long long limit_ns;
+    unsigned last;  // after this step the block waits for a tag that none writes (self test)
     unsigned tag;
 
     // The timer is read only now and then: a read takes about as long as the
     // message it waits for.
-    __device__ __forceinline__ bool poll(const ulonglong2* p, double& u) const
+    __device__ __forceinline__ bool poll(const ulonglong2* p, unsigned want, double& u) const
     {
         for (int n = 0; n < 256; ++n)
-            if (slot_load(p, tag, u))
+            if (slot_load(p, want, u))
                 return true;
         const unsigned long long t0 = globaltimer_ns();
-        for (unsigned n = 1; !slot_load(p, tag, u); ++n)
+        for (unsigned n = 1; !slot_load(p, want, u); ++n)
         {
             if (n % 64u != 0)
                 continue;
@@ -191,10 +192,11 @@ struct GridSum
         int bad = 0;
         if (w < np)
         {
+            const unsigned want = tag <= last ? tag : 0u;
             double acc = 0.0, u = 0.0;
             for (int i = threadIdx.x; i < G && !bad; i += np * 32)
             {
-                bad = poll(row + i * kPad, u) ? 0 : 1;
+                bad = poll(row + i * kPad, want, u) ? 0 : 1;
                 acc += u;
             }
             acc = warp_sum(acc);
@@ -231,7 +233,8 @@ __global__ void __launch_bounds__(kSingleThreads, 1) cg_single_kernel(SolveDesc 
     const Lat& L = d.L;
     const bool dag1 = d.dag_first != 0;
     const int beg = int(blockIdx.x) * d.ch, end = min(beg + d.ch, L.nsite);
-    GridSum gsum{reinterpret_cast<ulonglong2*>(d.part), sm, d.bar, d.timeout_ns, 0u};
+    GridSum gsum{reinterpret_cast<ulonglong2*>(d.part), sm, d.bar, d.timeout_ns,
+                 d.mute && blockIdx.x + 1 == gridDim.x ? 2u : ~0u, 0u};
     const long uo = long(d.rhs_conf[0]) * d.usz;
     const double2* const U64 = d.U64 + uo;
     const T* const U = MIXED ? reinterpret_cast<const T*>(d.U32 + uo) : reinterpret_cast<const T*>(U64);

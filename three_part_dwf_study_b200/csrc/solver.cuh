@@ -53,6 +53,7 @@ struct SolveDesc
     int* out_ru;
     GridBar* bar;
     unsigned long long timeout_ns;
+    unsigned mute;  // self test of the waits: sums waited for that are never sent (dwf_set_missing_sums)
     unsigned expected_blocks;  // normally gridDim.x
 };
 
