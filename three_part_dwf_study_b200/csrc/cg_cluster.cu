@@ -229,6 +229,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
                 if (s0 + j < Ls)
                     send_spinor(tonext + unsigned((f ? fT : 0) + (s0 + j) * ss) * 16u, plane, v[j], barnext + 16u * f);
     };
+    auto ran_out = [&] { quit.from(it + 1); };
     auto halo = [&](int f) {
         const unsigned b = hbar + 16u * f, ph = (par >> (kSlots + f)) & 1u;
         if (threadIdx.x == 0 && !bad)
@@ -241,15 +242,15 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
         if ((threadIdx.x & 31) == 0)
         {
             if (lo)
-                cl::wait(b, ph, d.timeout_ns, quit, it, bad);
+                cl::wait(b, ph, d.timeout_ns, bad, ran_out);
             if (hi)
-                cl::wait(b + 8u, ph, d.timeout_ns, quit, it, bad);
+                cl::wait(b + 8u, ph, d.timeout_ns, bad, ran_out);
         }
         __syncwarp();
         par ^= (1u << kSlots) << f;
     };
     auto total = [&](int slot) {
-        const double v = sum.get(slot, (par >> slot) & 1u, d.timeout_ns, quit, it, bad);
+        const double v = sum.get(slot, (par >> slot) & 1u, d.timeout_ns, bad, ran_out);
         par ^= 1u << slot;
         return v;
     };
@@ -306,7 +307,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
         for (int i = 0; i < kSlots + 4; ++i)
             cl::bar_init(bars + 8u * i, i < kSlots && rank + 1 == CS ? (d.mute >> i) & 1u : 0u);
         meet.init();
-        asm volatile("st.shared::cta.u32 [%0], 0;" ::"r"(quit.word) : "memory");
+        quit.init();
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cl::sync();

@@ -13,10 +13,11 @@
 // message into the same place needs data the receiver sends only after it has
 // read the last one (each solver says why at its phases).
 //
-// A wait that runs past the limit is noted in the waiting lane (`bad`) and in the CTA's
-// shared memory (Quit). The warps of a CTA may then hold different values of a sum,
-// so nothing that decides which barrier comes next is taken from a sum before all
-// threads know that none has; a CTA that gives up goes to the next check point (Meet).
+// A wait that runs past the limit is noted in the waiting lane (`bad`). The warps of
+// a CTA may then hold different values of a sum, so each solver's loop is laid out
+// such that warps on different ways meet at the same block barriers up to one that
+// tells all of them (by __syncthreads_or of `bad`, or Quit). The CTA then gives up and
+// goes to the next check point (Meet).
 #pragma once
 
 #include <cooperative_groups.h>
@@ -100,6 +101,17 @@ __device__ __forceinline__ bool bar_wait(unsigned bar, unsigned parity, unsigned
     return true;
 }
 
+// One lane's wait; a lane that is bad waits no more. ran_out() when it becomes bad.
+template <typename F>
+__device__ __forceinline__ void wait(unsigned bar, unsigned parity, unsigned long long limit_ns, int& bad, F ran_out)
+{
+    if (!bad && !bar_wait(bar, parity, limit_ns))
+    {
+        bad = 1;
+        ran_out();
+    }
+}
+
 // Cluster barrier (release / acquire at cluster scope).
 __device__ __forceinline__ void sync() { cg::this_cluster().sync(); }
 
@@ -109,38 +121,6 @@ __device__ __forceinline__ void sync_global()
 {
     __threadfence();
     cg::this_cluster().sync();
-}
-
-// The iteration from which a CTA gives up: one more than the iteration in which a
-// wait ran out first (shared memory, zero: none has). All threads read it between the
-// block barrier that starts an iteration and the next one; noted numbers lie beyond the
-// iteration then, so all get the same answer however late they read.
-struct Quit
-{
-    unsigned word;  // shared address
-
-    __device__ __forceinline__ void from(int it) const
-    {
-        unsigned old;
-        asm volatile("atom.shared::cta.cas.b32 %0, [%1], 0, %2;" : "=r"(old) : "r"(word), "r"(it) : "memory");
-    }
-    __device__ __forceinline__ bool at(int it) const
-    {
-        unsigned v;
-        asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(word) : "memory");
-        return v - 1u < unsigned(it);
-    }
-};
-
-// One lane's wait in iteration `it`. A lane that is bad waits no more.
-__device__ __forceinline__ void wait(unsigned bar, unsigned parity, unsigned long long limit_ns, const Quit& quit,
-                                     int it, int& bad)
-{
-    if (!bad && !bar_wait(bar, parity, limit_ns))
-    {
-        bad = 1;
-        quit.from(it + 1);
-    }
 }
 
 // Sum over the cluster of one value per thread, in three steps: part() leaves
@@ -174,15 +154,16 @@ struct Sum
     }
     // Thread 0 arms no more once it is bad (its barrier may still be in the phase it
     // armed last).
-    __device__ __forceinline__ double get(int slot, unsigned parity, unsigned long long limit_ns, const Quit& quit,
-                                          int it, int& bad) const
+    template <typename F>
+    __device__ __forceinline__ double get(int slot, unsigned parity, unsigned long long limit_ns, int& bad,
+                                          F ran_out) const
     {
         const int lane = threadIdx.x & 31;
         if (lane == 0 && !bad)
         {
             if (threadIdx.x == 0)
                 bar_expect(bar + 8u * slot, unsigned(CS) * 8u);
-            wait(bar + 8u * slot, parity, limit_ns, quit, it, bad);
+            wait(bar + 8u * slot, parity, limit_ns, bad, ran_out);
         }
         __syncwarp();
         return warp_sum(lane < CS ? tab[slot * kMaxCtas + lane] : 0.0);
@@ -206,7 +187,8 @@ __host__ __device__ constexpr size_t sum_bytes(int nslot)
 // has read its own word there, hence the number and not a flag. True: leave.
 //
 // The word and the count of check points passed lie in shared memory (8 bytes at
-// `word`): a register each would cost the solvers' loops spills. Thread 0 counts after
+// `word`), and a solver looks at left() after its loop instead of leaving from within:
+// a register or a way out of the loop more cost the even-odd kernel spills and 1.5 %. Thread 0 counts after
 // the barrier; every solver has a block barrier before its next check point.
 struct Meet
 {
@@ -229,7 +211,43 @@ struct Meet
             asm volatile("st.shared::cta.u32 [%0], %1;" ::"r"(word + 4u), "r"(n) : "memory");
         return v == n;
     }
+    // Whether the last check point said to leave (after a block barrier).
+    __device__ __forceinline__ bool left() const
+    {
+        unsigned n, v;
+        asm volatile("ld.volatile.shared::cta.v2.u32 {%0, %1}, [%2];" : "=r"(v), "=r"(n) : "r"(word) : "memory");
+        return n != 0 && v == n;
+    }
 };
+
+// The iteration from which a CTA gives up: one more than the iteration in which a
+// wait ran out first (shared memory, zero: none has). All threads read it between the
+// block barrier that starts an iteration and the next one; numbers noted meanwhile lie
+// beyond the iteration, so all get the same answer however late they read. In the
+// full-lattice CG 2 % faster than __syncthreads_or, whose result the barrier waits
+// for; in the even-odd kernel, short of registers, 1.5 % slower.
+struct Quit
+{
+    unsigned word;  // shared address
+
+    __device__ __forceinline__ void init() const  // by one thread, before the first cluster barrier
+    {
+        asm volatile("st.shared::cta.u32 [%0], %1;" ::"r"(word), "r"(0) : "memory");
+    }
+    __device__ __forceinline__ void from(int it) const
+    {
+        unsigned old;
+        asm volatile("atom.shared::cta.cas.b32 %0, [%1], 0, %2;" : "=r"(old) : "r"(word), "r"(it) : "memory");
+    }
+    __device__ __forceinline__ bool at(int it) const
+    {
+        unsigned v;
+        asm volatile("ld.volatile.shared::cta.u32 %0, [%1];" : "=r"(v) : "r"(word) : "memory");
+        return v - 1u < unsigned(it);
+    }
+};
+
+constexpr int kGaveUp = -2;  // state of a right-hand side whose CTA gave up (beside RHS_ACTIVE and the status codes)
 
 // After a check point that says to leave: all messages have been sent, those still on
 // their way land long before this returns (they take about a microsecond).

@@ -74,7 +74,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr size_t kClHead = (cl::sum_bytes(3) + 9 * 8 + 15) / 16 * 16;  // sum tables, mbarriers, Meet and Quit
+constexpr size_t kClHead = (cl::sum_bytes(3) + 8 * 8 + 15) / 16 * 16;  // sum tables, mbarriers, Meet
 
 struct ClDesc
 {
@@ -343,8 +343,10 @@ __device__ __forceinline__ ClPlace cl_place(const ClDesc& c, int rank)
 // own places, |r|^2 of them returned. Kept out of line: it runs once in tens of
 // iterations, and its FP64 temporaries must not take the loop's registers.
 template <int LT, int NL, bool PAD>
-__device__ __noinline__ double cl_reliable(const EoDesc& e, const ClDesc& c, int rank, int jr)
+__device__ __noinline__ double cl_reliable(const EoDesc& e, const ClDesc& c, int rank, int jr, const cl::Meet meet)
 {
+    if (meet(false, c.CS))
+        return -1.0;
     const SolveDesc& d = e.d;
     const Lat& L = d.L;
     const ClPlace w = cl_place<NL>(c, rank);
@@ -432,7 +434,6 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
     float2* const LK = reinterpret_cast<float2*>(ES + (EREG ? 0 : LT * int(blockDim.x)));  // links [even, odd][4][sites]
     const cl::Sum sum{tab, tab + 3 * cl::kMaxCtas, bars, CS, rank};
     const cl::Meet meet{bars + 7 * 8};
-    const cl::Quit quit{meet.word + 8u};
     // lane D q + i of warp w (D = 32 / NL): part q of 4-D site D w + i of each parity
     const ClPlace pl = cl_place<NL>(c, rank);
     const int q = pl.q, tl = pl.tl, k = pl.k, t = pl.t;
@@ -479,7 +480,8 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
     };
     // Parities of the barriers: bits 0-2 sums, 3 and 4 the halos of A and B.
     unsigned par = 0;
-    int bad = 0, it = 0;
+    int bad = 0;
+    auto ran_out = [] {};
     // Wait for the halo rows this thread reads from field A (f = 0) or B.
     auto halo = [&](int f) {
         const unsigned b = hbar + 16u * f, ph = (par >> (3 + f)) & 1u;
@@ -494,15 +496,15 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
         if ((threadIdx.x & 31) == 0)
         {
             if (lo)
-                cl::wait(b, ph, d.timeout_ns, quit, it, bad);
+                cl::wait(b, ph, d.timeout_ns, bad, ran_out);
             if (hi)
-                cl::wait(b + 8u, ph, d.timeout_ns, quit, it, bad);
+                cl::wait(b + 8u, ph, d.timeout_ns, bad, ran_out);
         }
         __syncwarp();
         par ^= 8u << f;
     };
     auto total = [&](int slot) {
-        const double v = sum.get(slot, (par >> slot) & 1u, d.timeout_ns, quit, it, bad);
+        const double v = sum.get(slot, (par >> slot) & 1u, d.timeout_ns, bad, ran_out);
         par ^= 1u << slot;
         return v;
     };
@@ -511,7 +513,6 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
         for (int i = 0; i < 7; ++i)
             cl::bar_init(bars + 8u * i, i < 3 && rank + 1 == CS ? (d.mute >> i) & 1u : 0u);
         meet.init();
-        asm volatile("st.shared::cta.u32 [%0], 0;" ::"r"(quit.word) : "memory");
         asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
     }
     cl::sync();
@@ -567,18 +568,17 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
             sum.send(2);
         const double bb = total(2);
         double rr = bb, rru = bb, cf = 0.0;
-        it = 0;
-        int ru = 0, stalls = 0;
+        int it = 0, ru = 0, stalls = 0;
         int state = (bb == 0.0 || persist::converged_now(d, rr, bb) || d.maxiter < 1) ? DWF_OK : RHS_ACTIVE;
         if (state == DWF_OK && !(bb == 0.0 || persist::converged_now(d, rr, bb)))
             state = DWF_NOT_CONVERGED;
 
+        if (__syncthreads_or(bad))
+            state = cl::kGaveUp;
         clk.start();
         // Between two reliable updates: p and r come from memory (p from field
-        // A's own places), e starts at zero. `gave` is the same in all threads of the
-        // CTA, and so is every value taken from a sum once it is false.
-        bool gave = __syncthreads_or(bad) != 0;
-        while (state == RHS_ACTIVE && !gave)
+        // A's own places), e starts at zero.
+        while (state == RHS_ACTIVE)
         {
             Spinor<float> p[LT], r[LT], ev[EREG ? LT : 1];
 #pragma unroll
@@ -591,7 +591,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 else
                     ev[EREG ? j : 0] = zero;
             }
-            bool want = false, zden = false;
+            bool want = false;
             do
             {
                 ++it;
@@ -604,8 +604,11 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 for (int j = 0; j < LT; ++j)
                     p[j] = persist::axpy(beta, p[j], r[j]);
                 store(0, p);
-                __syncthreads();
-                gave = quit.at(it);
+                if (__syncthreads_or(bad))
+                {
+                    state = cl::kGaveUp;
+                    break;
+                }
                 clk.mark(6);
                 // P1: y = M5^-1 H_eo p
                 halo(0);
@@ -632,8 +635,6 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                         for (int j = 0; j < LT; ++j)
                             yk[EREG ? j : 0] = z[j];
                 }
-                if (gave)
-                    break;
                 __syncthreads();
                 clk.mark(0);
                 // P2: t = M5 p - H_oe y, |t|^2
@@ -697,8 +698,11 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 __syncthreads();
                 clk.mark(3);
                 const double tt = total(1);
-                // ends the solve after this phase, e and r dropped
-                zden = tt == 0.0 || !isfinite(tt);
+                if (tt == 0.0 || !isfinite(tt))
+                {
+                    state = DWF_NOT_CONVERGED;
+                    break;
+                }
                 const float al = float(rr / tt);
                 clk.mark(2);
                 // P4: Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap; |r|^2
@@ -736,24 +740,25 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     sum.send(0);
                 clk.mark(4);
                 const double rn = total(0);
-                want = zden || rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
+                want = rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
                 cf = rn / rr;
-                rr = zden ? rr : rn;
+                rr = rn;
                 clk.mark(5);
             } while (!want);
-            // (a warp whose sum ran out may be at the next iteration's first barrier)
-            if (!gave)
+            // Warps of a CTA whose waits ran out may be here for the zero denominator, for
+            // the reliable update or not yet: the first meet the others at P4's barrier, then
+            // all at the one before P1.
+            if (state == cl::kGaveUp)
+                break;
+            if (state != RHS_ACTIVE)
             {
+                halo(1);  // the y rows on their way
                 __syncthreads();
-                gave = quit.at(it + 1);
             }
-            if (gave)
+            if (__syncthreads_or(bad))
+                state = cl::kGaveUp;
+            if (state != RHS_ACTIVE)
                 break;
-            if (zden)
-            {
-                state = DWF_NOT_CONVERGED;
-                break;
-            }
             // ---- reliable update in FP64: x += e, r = b - Dhat^dag Dhat x ----
 #pragma unroll
             for (int j = 0; j < LT; ++j)
@@ -766,18 +771,18 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     st_spinor(xj, gi, Spinor<double>{xo.s0 + de.s0, xo.s1 + de.s1});
                     FA[(s0 + j) * SS + own] = s2f4(p[j]);
                 }
-            if (meet(false, CS))
-            {
-                cl::settle();
-                return;
-            }
-            a0 = cl_reliable<LT, NL, PAD>(e, c, rank, jr);
+            a0 = cl_reliable<LT, NL, PAD>(e, c, rank, jr, meet);
+            bad |= a0 < 0.0;
             sum.part(2, a0);
             __syncthreads();
-            if (threadIdx.x < 32)
+            if (threadIdx.x < 32 && !bad)
                 sum.send(2);
             const double rt = total(2);
-            gave = __syncthreads_or(bad) != 0;
+            if (__syncthreads_or(bad))
+            {
+                state = cl::kGaveUp;
+                break;
+            }
             ru += 1;
             cf = cf * (rt / rr);
             stalls = (rt >= 0.5 * rru) ? stalls + 1 : 0;
@@ -789,6 +794,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 state = DWF_NOT_CONVERGED;
             clk.mark(5);
         }
+        const bool gave = state == cl::kGaveUp;
         if (gave && threadIdx.x == 0)
             raise_error(d.bar, DWF_TIMEOUT);
         clk.report();
@@ -800,7 +806,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
             d.out_ru[jr] = ru;
         }
         // the next right-hand side overwrites the fields and partials
-        if (meet(gave, CS))
+        if (meet.left() || meet(gave, CS))
         {
             cl::settle();
             return;
