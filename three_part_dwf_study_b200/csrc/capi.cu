@@ -37,22 +37,24 @@ using namespace dwfb;
 // 1331 / 1365 / 1354; 1.5 -> 1368 / 1387 / 1364; 2 -> 1385 / 1403 / 1377; 3 ->
 // 1404 / 1401 / 1393 (up to 5 iterations); 4 -> 1127 / 1150 / 1142 (up to 67:
 // past about 3x the full-lattice solve has to remove the Schur solution's low
-// modes). 2 keeps a margin below that edge. Where the grid-wide Schur kernel
-// runs (right-hand sides too large for a cluster) the same pair cost the
-// finite-volume study at 64x96x16 (1792 sources) 20 % (451.5 against 561.9
-// solves/s; 64x80x16: 719.6 against 706.5), so that path keeps factor 1 and
-// the mixed check solve.
+// modes). What a looser stop gains in time it loses in the solution, whose error
+// follows the Schur residual: with the cluster kernel's present form, 28 sources to
+// 1e-12 (FP64 check; ms a batch, mean error against a 3e-14 solve), factor 1 and 2:
+// 64x64x16 16.66, 6.3e-11 and 16.36, 1.3e-10; 62x94x16 25.1, 8.6e-11 and 24.6,
+// 1.8e-10; 48x48x24 19.4, 9.8e-11 and 19.1, 1.8e-10; 64x96x16 with 56 49.6, 8.1e-11
+// and 48.6, 1.7e-10 (grid-wide kernel, factor 1: 116, 5.3e-11: its updates every 16
+// iterations overshoot). So both kernels stop at the tolerance itself. The check solve
+// is the FP64 one after the cluster kernel (mixed: 1.4 % slower at these four) and
+// the mixed one after the grid-wide kernel (FP64 with factor 2 cost the finite-volume
+// study at 64x96x16, 1792 sources, 20 %).
 #ifndef DWFB_EO_SCHUR_TOL
-#define DWFB_EO_SCHUR_TOL 2.0       // cluster Schur kernel
+#define DWFB_EO_SCHUR_TOL 1.0
 #endif
 #ifndef DWFB_EO_POLISH_SOLVER
-#define DWFB_EO_POLISH_SOLVER DWF_SOLVER_CG64
-#endif
-#ifndef DWFB_EO_SCHUR_TOL_GRID
-#define DWFB_EO_SCHUR_TOL_GRID 1.0  // grid-wide Schur kernel
+#define DWFB_EO_POLISH_SOLVER DWF_SOLVER_CG64  // cluster Schur kernel
 #endif
 #ifndef DWFB_EO_POLISH_SOLVER_GRID
-#define DWFB_EO_POLISH_SOLVER_GRID DWF_SOLVER_MIXED
+#define DWFB_EO_POLISH_SOLVER_GRID DWF_SOLVER_MIXED  // grid-wide Schur kernel
 #endif
 #ifndef DWFB_PIPE_CHUNKS
 // Chunks of a host-buffer even-odd cluster batch (1 to 4). At 64x64x16 with 28
@@ -811,8 +813,7 @@ int propagators(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, dou
         // stopping rule |D^dag D x - D^dag src| <= rtol |D^dag src| decides.
         std::vector<int> eo_it, eo_ru;
         const bool clustered = eo_cluster_wave(c, nrhs) > 0;
-        const double schur_tol = (clustered ? DWFB_EO_SCHUR_TOL : DWFB_EO_SCHUR_TOL_GRID) * rtol;
-        st = propagators_eo(c, nrhs, conf_h, src, x, schur_tol, maxiter, eo_it, eo_ru);
+        st = propagators_eo(c, nrhs, conf_h, src, x, DWFB_EO_SCHUR_TOL * rtol, maxiter, eo_it, eo_ru);
         if (st)
             return st;
         // The reference's rule on the full normal equation, in FP64: where every
