@@ -341,8 +341,8 @@ int dwf_z4_digits(uint64_t seed, long n, signed char* out);
  * DWF_NOALLOC_MAX_LINKS = 2*Nt*Nx links; larger ones return DWF_BAD_ARG.
  * params->device selects (and leaves current) the GPU. The first call on a
  * device resolves the array's device address (kept for the process's life,
- * so no use across a cudaDeviceReset), so make that first call before any
- * stream capture. While another thread holds a capture open, that capture
+ * so no use across a cudaDeviceReset) and loads the code for every lattice, so
+ * make that first call before any stream capture. While another thread holds a capture open, that capture
  * must use cudaStreamCaptureModeThreadLocal or ...Relaxed: in global mode
  * CUDA forbids every other thread the synchronous read-back this call makes.
  * Calls share the array: calls whose GPU work overlaps race and must be

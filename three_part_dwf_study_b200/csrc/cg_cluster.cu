@@ -611,6 +611,19 @@ double grid_time(const Lat& L, bool mixed, int nrhs)
 
 }  // namespace
 
+cudaError_t load_cg_cluster64()
+{
+    for (int LT = 1; LT <= kMaxLt64; ++LT)
+        for (int NL = 1; NL <= 8; NL *= 2)
+        {
+            cudaFuncAttributes a;
+            const cudaError_t e = cudaFuncGetAttributes(&a, kernel_of(false, true, LT, NL));
+            if (e != cudaSuccess)
+                return e;
+        }
+    return cudaSuccess;
+}
+
 // The cluster shape with the least estimated time of an iteration over the whole
 // batch, if that beats the grid-wide kernels. An iteration takes about 1.4 us of
 // message and sum latencies (1.8 with the fifth dimension's shuffles), plus per

@@ -10,4 +10,8 @@ namespace dwfb {
 // d.bar is zeroed; d.part is not used.
 cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cudaStream_t stream, bool* taken);
 
+// Load the code of every FP64 domain-wall instance launch_cg_cluster may pick on the
+// current device.
+cudaError_t load_cg_cluster64();
+
 }  // namespace dwfb

@@ -60,7 +60,9 @@ void* g_base[kMaxDevices] = {};
 // name g_scratch is only a host-side stand-in, never a device address. The
 // address is resolved on the first call per device and kept for the life of
 // the process: a cudaDeviceReset of that device (which unloads the module)
-// leaves it stale, so the entry point must not be used across a device reset.
+// leaves it stale, so the entry point must not be used across a device reset. That
+// call also loads every kernel a later one may launch, whatever its lattice, operator
+// or solver kernel (loading takes device memory and is not allowed everywhere).
 int scratch_base(int dev, unsigned char** base)
 {
     if (dev < 0 || dev >= kMaxDevices)
@@ -70,6 +72,15 @@ int scratch_base(int dev, unsigned char** base)
     {
         void* p = nullptr;
         if (cudaGetSymbolAddress(&p, g_scratch) != cudaSuccess || !p)
+            return DWF_CUDA_ERROR;
+        cudaFuncAttributes a;
+        if (cudaFuncGetAttributes(&a, &links_kernel) != cudaSuccess ||
+            cudaFuncGetAttributes(&a, &dirac_kernel<true, double>) != cudaSuccess ||
+            cudaFuncGetAttributes(&a, &dirac_kernel<false, double>) != cudaSuccess ||
+            cudaFuncGetAttributes(&a, &residual_partials_kernel<true>) != cudaSuccess ||
+            cudaFuncGetAttributes(&a, &residual_partials_kernel<false>) != cudaSuccess ||
+            cudaFuncGetAttributes(&a, &residual_finish_kernel) != cudaSuccess ||
+            load_cg_cluster64() != cudaSuccess || load_single64() != cudaSuccess)
             return DWF_CUDA_ERROR;
         g_base[dev] = p;
     }

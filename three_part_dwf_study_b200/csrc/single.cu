@@ -406,6 +406,13 @@ __global__ void __launch_bounds__(kSingleThreads, 1) cg_single_kernel(SolveDesc 
 
 size_t single_part_doubles(int nsm) { return size_t(4) * GridSum::kPad * size_t(nsm); }
 
+cudaError_t load_single64()
+{
+    cudaFuncAttributes a;
+    const cudaError_t e = cudaFuncGetAttributes(&a, &cg_single_kernel<false, true>);
+    return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, &cg_single_kernel<false, false>);
+}
+
 cudaError_t launch_single(SolveDesc& d, bool mixed, int nsm, cudaStream_t stream)
 {
     // one block per SM at most (the blocks wait on one another); one site per

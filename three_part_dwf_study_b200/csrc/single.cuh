@@ -15,4 +15,7 @@ size_t single_part_doubles(int nsm);
 // d.ch and d.expected_blocks.
 cudaError_t launch_single(SolveDesc& d, bool mixed, int nsm, cudaStream_t stream);
 
+// Load the code of launch_single's FP64 instances on the current device.
+cudaError_t load_single64();
+
 }  // namespace dwfb
