@@ -413,7 +413,7 @@ int dwf_set_eo_kernel(dwf_ctx* ctx, int kernel);
 
 /* Per-phase device timers of the even-odd solver kernel (grid-wide kernel: block 0's
  * view, each phase including the grid barrier that ends it; cluster kernel: the
- * right-hand side that took longest): enable (1) allocates and
+ * right-hand side that took longest in each launch): enable (1) allocates and
  * zeroes them, 0 frees them (off by default: no cost). dwf_eo_phase_times
  * returns accumulated ms and counts for the phases 0 hop + M5^-1, 1 M5 - H
  * (|t|^2), 2 alpha reduction, 3 adjoint hop + M5^-1, 4 adjoint combine and

@@ -101,6 +101,13 @@ int ensure_eo(dwf_ctx* c, int nrhs)
     return DWF_OK;
 }
 
+// Adds a cluster launch's phase times [16, 32) to the totals [0, 16) and clears them.
+__global__ void eo_phase_add_kernel(unsigned long long* ph)
+{
+    ph[threadIdx.x] += ph[16 + threadIdx.x];
+    ph[16 + threadIdx.x] = 0;
+}
+
 constexpr size_t kGraphCache = 16;
 
 // Run `body` (stream work only) through a CUDA graph cached under `key`:
@@ -267,6 +274,12 @@ int propagators_eo(dwf_ctx* c, int nrhs, const int* conf_h, const double2* src, 
                     return s2 ? s2 : ctx_fail(c, DWF_CUDA_ERROR, "even-odd cluster solver: launch failed");
                 CK(cudaEventRecordWithFlags(c->ev1, c->stream, cudaEventRecordExternal));
                 c->launches += 1;
+                if (c->eo_phase)
+                {
+                    eo_phase_add_kernel<<<1, 16, 0, c->stream>>>(c->eo_phase);
+                    CK(cudaGetLastError());
+                    c->launches += 1;
+                }
                 return reconstruct();
             });
             if (st)
@@ -370,7 +383,7 @@ int dwf_eo_phase_profile(dwf_ctx* c, int enable)
         return DWF_BAD_ARG;
     CK(cudaSetDevice(c->device));
     if (enable && !c->eo_phase)
-        CK(cudaMalloc(&c->eo_phase, 16 * sizeof(unsigned long long)));
+        CK(cudaMalloc(&c->eo_phase, 32 * sizeof(unsigned long long)));
     if (!enable && c->eo_phase)
     {
         CK(cudaStreamSynchronize(c->stream));
@@ -378,7 +391,7 @@ int dwf_eo_phase_profile(dwf_ctx* c, int enable)
         c->eo_phase = nullptr;
     }
     if (c->eo_phase)
-        CK(cudaMemsetAsync(c->eo_phase, 0, 16 * sizeof(unsigned long long), c->stream));
+        CK(cudaMemsetAsync(c->eo_phase, 0, 32 * sizeof(unsigned long long), c->stream));
     return DWF_OK;
 }
 

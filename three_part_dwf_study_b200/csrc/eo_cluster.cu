@@ -280,7 +280,8 @@ __device__ __forceinline__ Spinor<double> cl_m5_64(const double2* __restrict__ f
 }
 
 // Phase timer of the cluster's first thread, kept per right-hand side in shared
-// memory; the longest right-hand side's times and counts are reported.
+// memory; the longest right-hand side's times and counts of this launch are reported
+// in ph[16, 32), which eo_phase_add_kernel adds to the running totals.
 struct ClClock
 {
     unsigned long long* ph;  // null: off
@@ -308,8 +309,8 @@ struct ClClock
             return;
         for (int k = 0; k < 7; ++k)
         {
-            atomicMax(ph + k, sm[1 + k]);
-            atomicMax(ph + 8 + k, sm[8 + k]);
+            atomicMax(ph + 16 + k, sm[1 + k]);
+            atomicMax(ph + 24 + k, sm[8 + k]);
         }
     }
 };
