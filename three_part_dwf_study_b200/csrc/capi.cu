@@ -624,14 +624,17 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
     int st = DWF_OK;
     bool clustered = false;
     CK(cudaMemsetAsync(c->bar, 0, sizeof(GridBar), c->stream));
-    CK(cudaEventRecord(c->ev0, c->stream));
-    CK(launch_cg_cluster(d, mixed, c->device, c->nsm, c->stream, &clustered));
+    // (ev0 right before each launch: host work after it would count as the solver's)
+    CK(launch_cg_cluster(d, mixed, c->device, c->nsm, c->stream, c->ev0, &clustered));
     if (!clustered && nrhs == 1)
     {
+        if (!c->single_loaded[mixed])
+            CK(load_single(mixed));
+        c->single_loaded[mixed] = true;
         if ((st = ensure_part(c, single_part_doubles(c->nsm))))
             return st;
         d.part = c->w_part;
-        CK(launch_single(d, mixed, c->nsm, c->stream));
+        CK(launch_single(d, mixed, c->nsm, c->stream, c->ev0));
     }
     else if (!clustered)
     {
@@ -651,6 +654,7 @@ int launch_solver(dwf_ctx* c, bool mixed, int op, int nrhs, const double2* b, do
         d.part = c->w_part;
         d.expected_blocks = unsigned(grid);
         void* args[] = {&d};
+        CK(cudaEventRecord(c->ev0, c->stream));
         CK(cudaLaunchCooperativeKernel(fn, dim3(grid), dim3(kSolverThreads), args, smem, c->stream));
     }
     CK(cudaEventRecord(c->ev1, c->stream));

@@ -633,7 +633,8 @@ cudaError_t load_cg_cluster64()
 // an iteration, FP64): Wilson 32x32 2.6 at 2 to 7 CTAs' rows each, 3.1 with two CTAs;
 // 12x10x6 3.3 / 3.9 / 4.7 at LT 1 / 2 / 3; 24x20x10 4.7 at LT 2, 5.2 at 3; 48x40 with 16
 // right-hand sides 2.8 (grid-wide 18); 40x40x8 5.2 (grid-wide 5.6).
-cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cudaStream_t stream, bool* taken)
+cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cudaStream_t stream,
+                              cudaEvent_t before, bool* taken)
 {
     *taken = false;
     const Lat& L = d.L;
@@ -688,7 +689,10 @@ cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cud
     cudaLaunchAttribute attr;
     config(best, std::min(best.resident, d.nrhs), stream, cfg, attr);
     void* args[] = {&d, &g};
-    const cudaError_t e = cudaLaunchKernelExC(&cfg, best.fn, args);
+    cudaError_t e = before ? cudaEventRecord(before, stream) : cudaSuccess;
+    if (e != cudaSuccess)
+        return e;
+    e = cudaLaunchKernelExC(&cfg, best.fn, args);
     *taken = e == cudaSuccess;
     return e;
 }

@@ -45,6 +45,7 @@ struct dwf_ctx
     std::map<int, DslashChoice> dslash_tuned;
     // CUDA events bracketing each persistent solver launch on `stream`
     cudaEvent_t ev0 = nullptr, ev1 = nullptr;
+    bool single_loaded[2] = {};  // code of cg_single_kernel: FP64, mixed
     cudaEvent_t join_ev[2] = {};  // ordering against a caller's stream (dwf_stream_enter / _leave)
     // device time of solver launches: full lattice, even-odd (either kernel),
     // even-odd cluster kernel alone

@@ -80,7 +80,7 @@ int scratch_base(int dev, unsigned char** base)
             cudaFuncGetAttributes(&a, &residual_partials_kernel<true>) != cudaSuccess ||
             cudaFuncGetAttributes(&a, &residual_partials_kernel<false>) != cudaSuccess ||
             cudaFuncGetAttributes(&a, &residual_finish_kernel) != cudaSuccess ||
-            load_cg_cluster64() != cudaSuccess || load_single64() != cudaSuccess)
+            load_cg_cluster64() != cudaSuccess || load_single(false) != cudaSuccess)
             return DWF_CUDA_ERROR;
         g_base[dev] = p;
     }
@@ -183,8 +183,8 @@ extern "C" int dwf_cg_noalloc(const dwf_params* p, int op, const double* theta_d
         return DWF_CUDA_ERROR;
     d.part = part;
     bool clustered = false;
-    if (launch_cg_cluster(d, false, p->device, nsm, stream, &clustered) != cudaSuccess ||
-        (!clustered && launch_single(d, false, nsm, stream) != cudaSuccess))
+    if (launch_cg_cluster(d, false, p->device, nsm, stream, nullptr, &clustered) != cudaSuccess ||
+        (!clustered && launch_single(d, false, nsm, stream, nullptr) != cudaSuccess))
         return DWF_CUDA_ERROR;
 
     // FP64 true residual |b - A x| / |b| with the scratch temporary t

@@ -406,14 +406,18 @@ __global__ void __launch_bounds__(kSingleThreads, 1) cg_single_kernel(SolveDesc 
 
 size_t single_part_doubles(int nsm) { return size_t(4) * GridSum::kPad * size_t(nsm); }
 
-cudaError_t load_single64()
+cudaError_t load_single(bool mixed)
 {
     cudaFuncAttributes a;
-    const cudaError_t e = cudaFuncGetAttributes(&a, &cg_single_kernel<false, true>);
-    return e != cudaSuccess ? e : cudaFuncGetAttributes(&a, &cg_single_kernel<false, false>);
+    const cudaError_t e = mixed ? cudaFuncGetAttributes(&a, &cg_single_kernel<true, true>)
+                                : cudaFuncGetAttributes(&a, &cg_single_kernel<false, true>);
+    if (e != cudaSuccess)
+        return e;
+    return mixed ? cudaFuncGetAttributes(&a, &cg_single_kernel<true, false>)
+                 : cudaFuncGetAttributes(&a, &cg_single_kernel<false, false>);
 }
 
-cudaError_t launch_single(SolveDesc& d, bool mixed, int nsm, cudaStream_t stream)
+cudaError_t launch_single(SolveDesc& d, bool mixed, int nsm, cudaStream_t stream, cudaEvent_t before)
 {
     // one block per SM at most (the blocks wait on one another); one site per
     // thread while a block's share fits, in blocks of at least 128 threads
@@ -428,6 +432,8 @@ cudaError_t launch_single(SolveDesc& d, bool mixed, int nsm, cudaStream_t stream
                            : (one ? reinterpret_cast<const void*>(&cg_single_kernel<false, true>)
                                   : reinterpret_cast<const void*>(&cg_single_kernel<false, false>));
     cudaError_t e = cudaMemsetAsync(d.part, 0, single_part_doubles(d.nch) * sizeof(double), stream);
+    if (e == cudaSuccess && before)
+        e = cudaEventRecord(before, stream);
     if (e != cudaSuccess)
         return e;
     void* args[] = {&d};
