@@ -149,9 +149,10 @@ int dwf_apply(dwf_ctx* ctx, int op, int conf, const double* in, double* out, int
 int dwf_apply_dev(dwf_ctx* ctx, int op, int conf, const void* in_dev, void* out_dev, int nrhs,
                   int precision);
 
-/* Order the context's stream behind what `stream` (a cudaStream_t of the same
- * device, as void*) holds so far, and `stream` behind what the context's stream
- * holds: around any _dev call. dwf_apply_on is dwf_apply_dev between the two. */
+/* Order the context's stream behind what `stream` (a cudaStream_t of the context's
+ * device, as void*; NULL: that device's default stream) holds so far, and `stream`
+ * behind what the context's stream holds: around any _dev call. dwf_apply_on is
+ * dwf_apply_dev between the two. All three make the context's device current. */
 int dwf_stream_enter(dwf_ctx* ctx, void* stream);
 int dwf_stream_leave(dwf_ctx* ctx, void* stream);
 int dwf_apply_on(dwf_ctx* ctx, int op, int conf, const void* in_dev, void* out_dev, int nrhs,

@@ -1140,6 +1140,7 @@ int dwf_stream_enter(dwf_ctx* c, void* stream)
 {
     if (!c)
         return DWF_BAD_ARG;
+    CK(cudaSetDevice(c->device));  // NULL is the current device's default stream
     CK(cudaEventRecord(c->join_ev[0], static_cast<cudaStream_t>(stream)));
     CK(cudaStreamWaitEvent(c->stream, c->join_ev[0], 0));
     return DWF_OK;
@@ -1149,6 +1150,7 @@ int dwf_stream_leave(dwf_ctx* c, void* stream)
 {
     if (!c)
         return DWF_BAD_ARG;
+    CK(cudaSetDevice(c->device));
     CK(cudaEventRecord(c->join_ev[1], c->stream));
     CK(cudaStreamWaitEvent(static_cast<cudaStream_t>(stream), c->join_ev[1], 0));
     return DWF_OK;
@@ -1158,7 +1160,6 @@ int dwf_apply_on(dwf_ctx* c, int op, int conf, const void* in, void* out, int nr
 {
     if (!c || !in || !out)
         return DWF_BAD_ARG;
-    CK(cudaSetDevice(c->device));
     int st = dwf_stream_enter(c, stream);
     if (st)
         return st;
