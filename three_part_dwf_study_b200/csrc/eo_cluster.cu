@@ -825,11 +825,14 @@ namespace {
     DWFB_CL_PADS(X, 1, 2, er, mt) DWFB_CL_PADS(X, 2, 2, er, mt) DWFB_CL_PADS(X, 3, 2, er, mt)     \
     DWFB_CL_PADS(X, 4, 2, er, mt) DWFB_CL_PADS(X, 5, 2, er, mt) DWFB_CL_PADS(X, 6, 2, er, mt)     \
     DWFB_CL_PADS(X, 7, 2, er, mt) DWFB_CL_PADS(X, 8, 2, er, mt)
-#define DWFB_CL_FORM4(X, er, mt)                                                                  \
-    DWFB_CL_PADS(X, 1, 4, er, mt) DWFB_CL_PADS(X, 2, 4, er, mt) DWFB_CL_PADS(X, 3, 4, er, mt)     \
-    DWFB_CL_PADS(X, 4, 4, er, mt) DWFB_CL_PADS(X, 5, 4, er, mt) DWFB_CL_PADS(X, 6, 4, er, mt)
-#define DWFB_CL_KERNELS(X) \
-    DWFB_CL_FORM2(X, true, 256) DWFB_CL_FORM2(X, false, 384) DWFB_CL_FORM4(X, true, 512) DWFB_CL_FORM4(X, false, 768)
+// Four threads per site only where two cannot (cl_shape takes the first form that
+// fits): Ls > 16, and of the smaller Ls the two below, whose links and e take a little
+// less shared memory in CTAs of one or two long rows.
+#define DWFB_CL_KERNELS(X)                                                                      \
+    DWFB_CL_FORM2(X, true, 256) DWFB_CL_FORM2(X, false, 384)                                    \
+    DWFB_CL_PADS(X, 5, 4, true, 512) DWFB_CL_PADS(X, 6, 4, true, 512)                           \
+    X(3, 4, false, false, 768) X(4, 4, true, false, 768)                                        \
+    DWFB_CL_PADS(X, 5, 4, false, 768) DWFB_CL_PADS(X, 6, 4, false, 768)
 
 struct ClShape
 {
