@@ -19,13 +19,11 @@
 // stopping rule and count for Wilson). Mixed: FP32 iterations with FP64 reliable
 // updates as in cg_mixed_kernel, x, b and the FP64 temporaries in global memory.
 #include <algorithm>
-#include <map>
-#include <mutex>
-#include <tuple>
 #include <type_traits>
 
 #include "cg_cluster.cuh"
 #include "cluster.cuh"
+#include "cluster_launch.cuh"
 #include "persist.cuh"
 
 namespace dwfb {
@@ -531,13 +529,6 @@ namespace {
 
 constexpr size_t kSmemMax = 227 * 1024;
 
-struct Shape
-{
-    int CS = 0, R = 0, NL = 0, LT = 0, threads = 0, resident = 0;
-    size_t smem = 0;
-    const void* fn = nullptr;
-};
-
 // Slices per thread up to which r, the iterate and the temporaries stay in 128 registers.
 constexpr int kMaxLt32 = 6, kMaxLt64 = 3;
 
@@ -555,47 +546,6 @@ const void* kernel_of(bool mixed, bool fifth, int LT, int NL)
 #undef DWFB_CGC_NL
 #undef DWFB_CGC
     return nullptr;
-}
-
-void config(const Shape& s, int clusters, cudaStream_t stream, cudaLaunchConfig_t& cfg, cudaLaunchAttribute& attr)
-{
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = unsigned(s.CS);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg = cudaLaunchConfig_t{};
-    cfg.gridDim = dim3(unsigned(s.CS * clusters));
-    cfg.blockDim = dim3(unsigned(s.threads));
-    cfg.dynamicSmemBytes = s.smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-}
-
-// Clusters of this shape resident at once (0: none), queried once per device and shape.
-int resident_clusters(const Shape& s, int device)
-{
-    using Key = std::tuple<int, const void*, int, int, size_t>;
-    static std::map<Key, int> known;
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lock(mu);
-    const Key key(device, s.fn, s.CS, s.threads, s.smem);
-    const auto it = known.find(key);
-    if (it != known.end())
-        return it->second;
-    int n = 0;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr;
-    config(s, 1, nullptr, cfg, attr);
-    if (cudaFuncSetAttribute(s.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kSmemMax)) != cudaSuccess ||
-        cudaFuncSetAttribute(s.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, s.fn, &cfg) != cudaSuccess)
-    {
-        cudaGetLastError();
-        n = 0;
-    }
-    known[key] = n;
-    return n;
 }
 
 // Estimated time (us) of an iteration over the whole batch on the grid-wide kernels
@@ -640,7 +590,7 @@ cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cud
     const Lat& L = d.L;
     const bool fifth = L.fifth != 0;
     const int words = mixed ? 1 : 2;
-    Shape best;
+    ClusterLaunch best;
     double least = grid_time(L, mixed, d.nrhs);
     for (int R = L.Nt; R >= 1; --R)
     {
@@ -651,7 +601,7 @@ cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cud
             continue;  // fewer rows per CTA with as many CTAs
         for (int NL = 1; NL <= 8; NL *= 2)
         {
-            Shape s;
+            ClusterLaunch s;
             s.R = R;
             s.CS = CS;
             s.NL = NL;
@@ -668,7 +618,7 @@ cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cud
             if (s.smem > kSmemMax)
                 continue;
             s.fn = kernel_of(mixed, fifth, s.LT, NL);
-            if (!s.fn || (s.resident = resident_clusters(s, device)) < 1)
+            if (!s.fn || (s.resident = resident_clusters(s, device, kSmemMax)) < 1)
                 continue;
             const int used = std::min(s.resident, d.nrhs);
             const double share = std::max(1.0, double(used) * CS / nsm);
@@ -687,7 +637,7 @@ cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cud
     CgGeo g{best.CS, best.R, (best.R + 2) * L.Nx};
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
-    config(best, std::min(best.resident, d.nrhs), stream, cfg, attr);
+    best.config(std::min(best.resident, d.nrhs), stream, cfg, attr);
     void* args[] = {&d, &g};
     cudaError_t e = before ? cudaEventRecord(before, stream) : cudaSuccess;
     if (e != cudaSuccess)

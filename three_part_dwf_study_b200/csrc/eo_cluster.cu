@@ -58,12 +58,10 @@
 // residual of the Schur normal equation from x + e when the FP32 residual has
 // fallen by delta^2 since the last one, or convergence is in sight.
 #include <algorithm>
-#include <map>
-#include <mutex>
-#include <tuple>
 #include <vector>
 
 #include "cluster.cuh"
+#include "cluster_launch.cuh"
 #include "context.cuh"
 #include "eo.cuh"
 #include "persist.cuh"
@@ -834,12 +832,10 @@ namespace {
     X(3, 4, false, false, 768) X(4, 4, true, false, 768)                                        \
     DWFB_CL_PADS(X, 5, 4, false, 768) DWFB_CL_PADS(X, 6, 4, false, 768)
 
-struct ClShape
+struct ClShape : ClusterLaunch
 {
-    int CS = 0, R = 0, NL = 0, LT = 0, threads = 0, maxt = 0, resident = 0;
+    int maxt = 0;
     bool ereg = false;
-    size_t smem = 0;
-    const void* fn = nullptr;
 };
 
 size_t cl_smem_bytes(const Lat& L, const ClShape& s)
@@ -859,50 +855,6 @@ const void* cl_kernel(const ClShape& s, bool pad)
     DWFB_CL_KERNELS(DWFB_CL_PICK)
 #undef DWFB_CL_PICK
     return nullptr;
-}
-
-void cl_config(const ClShape& sh, int clusters, cudaStream_t stream, cudaLaunchConfig_t& cfg,
-               cudaLaunchAttribute& attr)
-{
-    attr.id = cudaLaunchAttributeClusterDimension;
-    attr.val.clusterDim.x = unsigned(sh.CS);
-    attr.val.clusterDim.y = 1;
-    attr.val.clusterDim.z = 1;
-    cfg = cudaLaunchConfig_t{};
-    cfg.gridDim = dim3(unsigned(sh.CS * clusters));
-    cfg.blockDim = dim3(unsigned(sh.threads));
-    cfg.dynamicSmemBytes = sh.smem;
-    cfg.stream = stream;
-    cfg.attrs = &attr;
-    cfg.numAttrs = 1;
-}
-
-// Clusters of this shape resident at once on the device (kernel attributes set
-// on the way), queried once per device and shape, so that a later call, the one
-// a stream capture records, issues the launch alone. 0: none.
-int cl_resident(const ClShape& sh, int device)
-{
-    using Key = std::tuple<int, const void*, int, int, size_t>;
-    static std::map<Key, int> known;
-    static std::mutex mu;
-    std::lock_guard<std::mutex> lock(mu);
-    const Key key(device, sh.fn, sh.CS, sh.threads, sh.smem);
-    const auto it = known.find(key);
-    if (it != known.end())
-        return it->second;
-    int n = 0;
-    cudaLaunchConfig_t cfg;
-    cudaLaunchAttribute attr;
-    cl_config(sh, 1, nullptr, cfg, attr);
-    if (cudaFuncSetAttribute(sh.fn, cudaFuncAttributeMaxDynamicSharedMemorySize, int(kClSmemMax)) != cudaSuccess ||
-        cudaFuncSetAttribute(sh.fn, cudaFuncAttributeNonPortableClusterSizeAllowed, 1) != cudaSuccess ||
-        cudaOccupancyMaxActiveClusters(&n, sh.fn, &cfg) != cudaSuccess)
-    {
-        cudaGetLastError();
-        n = 0;
-    }
-    known[key] = n;
-    return n;
 }
 
 // Cluster shape for a batch: the rows per CTA for which the estimated time of an
@@ -944,7 +896,7 @@ ClShape cl_shape(const dwf_ctx* c, int nrhs)
             if (sh.threads > sh.maxt || sh.smem > kClSmemMax)
                 continue;
             sh.fn = cl_kernel(sh, sh.NL * sh.LT != L.Ls);
-            if (!sh.fn || (sh.resident = cl_resident(sh, c->device)) < 1)
+            if (!sh.fn || (sh.resident = resident_clusters(sh, c->device, kClSmemMax)) < 1)
                 continue;
             const int used = std::min(sh.resident, nrhs);
             const double share = std::max(1.0, double(used) * sh.CS / c->nsm);
@@ -1015,7 +967,7 @@ int launch_eo_cluster(dwf_ctx* c, EoDesc& e, bool* launched, bool dry, int* wave
     cd.delta = 0.02;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;
-    cl_config(sh, std::min(sh.resident, e.d.nrhs), c->stream, cfg, attr);
+    sh.config(std::min(sh.resident, e.d.nrhs), c->stream, cfg, attr);
     void* args[] = {&e, &cd};
     if (cudaLaunchKernelExC(&cfg, sh.fn, args) != cudaSuccess)
         return ctx_fail(c, DWF_CUDA_ERROR, "even-odd cluster solver: launch failed");
