@@ -34,7 +34,7 @@ namespace cg = cooperative_groups;
 
 constexpr int kThreads = 512;
 constexpr int kSlots = 4;  // sums: |r|^2, |t|^2, |b|^2 and the replaced |r|^2
-constexpr size_t kHead = (cl::sum_bytes(kSlots) + (kSlots + 6) * 8 + 15) / 16 * 16;
+constexpr size_t kHead = cl::head_bytes(cl::sum_bytes(kSlots) + (kSlots + 6) * 8);
 
 struct CgGeo
 {
@@ -165,7 +165,7 @@ __global__ void __launch_bounds__(kThreads, 1) cg_cluster_kernel(const __grid_co
     const int rows = min(g.R, L.Nt - rank * g.R);
     const int prev = (rank + CS - 1) % CS, next = (rank + 1) % CS;
     const int prows = min(g.R, L.Nt - prev * g.R);
-    extern __shared__ __align__(16) unsigned char cg_smem[];
+    extern __shared__ __align__(128) unsigned char cg_smem[];
     double* const tab = reinterpret_cast<double*>(cg_smem);
     const unsigned bars = cl::smem_addr(cg_smem + cl::sum_bytes(kSlots));  // sums, then halos [p, t][prev, next]
     const unsigned hbar = bars + kSlots * 8;

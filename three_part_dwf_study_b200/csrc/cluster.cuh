@@ -169,6 +169,12 @@ struct Sum
         return warp_sum(lane < CS ? tab[slot * kMaxCtas + lane] : 0.0);
     }
 };
+// The solvers' fields begin at a multiple of 128 bytes behind the tables and
+// barriers: a warp's 16-byte words then cover whole lines. FP64 CG at 24x20x10 / 32x32x8
+// with 28 right-hand sides: 4.55 / 10.5 us an iteration there, 4.55 / 10.8 at 64 past
+// it, 4.77 / 11.5 at 32, 5.02 / 11.5 to 12.4 at 16 and 80.
+__host__ __device__ constexpr size_t head_bytes(size_t n) { return (n + 127) / 128 * 128; }
+
 __host__ __device__ constexpr size_t sum_bytes(int nslot)
 {
     return size_t(nslot) * (kMaxCtas + kMaxWarps) * sizeof(double);
@@ -224,8 +230,8 @@ struct Meet
 // wait ran out first (shared memory, zero: none has). All threads read it between the
 // block barrier that starts an iteration and the next one; numbers noted meanwhile lie
 // beyond the iteration, so all get the same answer however late they read. In the
-// full-lattice CG 2 % faster than __syncthreads_or, whose result the barrier waits
-// for; in the even-odd kernel, short of registers, 1.5 % slower.
+// full-lattice CG 1.5 % faster (32x32 Wilson) than __syncthreads_or, whose result the
+// barrier waits for.
 struct Quit
 {
     unsigned word;  // shared address

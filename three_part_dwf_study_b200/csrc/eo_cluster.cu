@@ -72,7 +72,7 @@ namespace {
 
 namespace cg = cooperative_groups;
 
-constexpr size_t kClHead = (cl::sum_bytes(3) + 8 * 8 + 15) / 16 * 16;  // sum tables, mbarriers, Meet
+constexpr size_t kClHead = cl::head_bytes(cl::sum_bytes(3) + 8 * 8);  // sum tables, mbarriers, Meet
 
 struct ClDesc
 {
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
     const int prev = (rank + CS - 1) % CS, next = (rank + 1) % CS;
     const int prows = min(c.R, c.Nt - prev * c.R);
     __shared__ unsigned long long clk_sm[15];
-    extern __shared__ __align__(16) unsigned char cl_smem[];
+    extern __shared__ __align__(128) unsigned char cl_smem[];
     double* const tab = reinterpret_cast<double*>(cl_smem);
     const unsigned bars = cl::smem_addr(cl_smem + cl::sum_bytes(3));  // sums, then halos [A, B][from prev, next]
     const unsigned hbar = bars + 3 * 8;
