@@ -590,25 +590,25 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 else
                     ev[EREG ? j : 0] = zero;
             }
-            bool want = false;
-            do
-            {
-                ++it;
-                // P5 of the iteration before: p = r + beta p
-                // (EREG) y and t at the own places, kept from the phase that forms them
-                // for the phases that read them: a quarter of the hops' loads
-                Spinor<float> yk[EREG ? LT : 1], tk[EREG ? LT : 1];
+            // P5 of the iteration before
+            auto direction = [&] {
                 const float beta = float(cf);
 #pragma unroll
                 for (int j = 0; j < LT; ++j)
                     p[j] = persist::axpy(beta, p[j], r[j]);
                 store(0, p);
-                if (__syncthreads_or(bad))
-                {
-                    state = cl::kGaveUp;
-                    break;
-                }
-                clk.mark(6);
+            };
+            direction();
+            // One barrier ends every iteration, whether it goes on or not, and tells all
+            // warps whether a wait of one of them ran out.
+            bool lost = __syncthreads_or(bad) != 0, want = lost, zden = false;
+            clk.mark(6);
+            while (!want)
+            {
+                ++it;
+                // (EREG) y and t at the own places, kept from the phase that forms them
+                // for the phases that read them: a quarter of the hops' loads
+                Spinor<float> yk[EREG ? LT : 1], tk[EREG ? LT : 1];
                 // P1: y = M5^-1 H_eo p
                 halo(0);
                 {
@@ -697,11 +697,7 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                 __syncthreads();
                 clk.mark(3);
                 const double tt = total(1);
-                if (tt == 0.0 || !isfinite(tt))
-                {
-                    state = DWF_NOT_CONVERGED;
-                    break;
-                }
+                zden = tt == 0.0 || !isfinite(tt);  // ends the solve, e and r dropped
                 const float al = float(rr / tt);
                 clk.mark(2);
                 // P4: Ap = M5^dag t - H^dag_oe y; e += alpha p; r -= alpha Ap; |r|^2
@@ -739,23 +735,18 @@ __global__ void __launch_bounds__(MAXT, 1) cg_eo_cluster_kernel(const __grid_con
                     sum.send(0);
                 clk.mark(4);
                 const double rn = total(0);
-                want = rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
+                want = zden || rn < c.delta * c.delta * rru || persist::converged_now(d, rn, bb) || it == d.maxiter;
                 cf = rn / rr;
-                rr = rn;
+                rr = zden ? rr : rn;
                 clk.mark(5);
-            } while (!want);
-            // Warps of a CTA whose waits ran out may be here for the zero denominator, for
-            // the reliable update or not yet: the first meet the others at P4's barrier, then
-            // all at the one before P1.
-            if (state == cl::kGaveUp)
-                break;
-            if (state != RHS_ACTIVE)
-            {
-                halo(1);  // the y rows on their way
-                __syncthreads();
+                if (!want)
+                    direction();
+                lost = __syncthreads_or(bad) != 0;
+                want = want || lost;
+                clk.mark(6);
             }
-            if (__syncthreads_or(bad))
-                state = cl::kGaveUp;
+            if (lost || zden)
+                state = lost ? cl::kGaveUp : DWF_NOT_CONVERGED;
             if (state != RHS_ACTIVE)
                 break;
             // ---- reliable update in FP64: x += e, r = b - Dhat^dag Dhat x ----
