@@ -985,6 +985,10 @@ def impl_ours(args):
                 "alg_bytes_per_launch": alg_bytes / max(1, nkern),
                 "kernel_ms_per_launch": kernel_launch_s * 1e3,
                 "kernel_share_of_step": kern_s / t_mixed}
+    if eo_kernel_name.startswith("cg_eo_cluster"):
+        # its fields stay on chip: the bytes its phases use, as a share of what HBM could
+        # have delivered, may exceed 1; what it moved is `traffic`
+        roofline["counted"] = "operand bytes of the phases, held on chip (not HBM traffic)"
 
     if use_learned:
         # the dominant kernel is then the tensor-core network layer

@@ -72,3 +72,28 @@ def test_full_lattice_solvers(T, Nt, Nx, Ls, n, solver):
 
     check(d, solve, (1, 2, 4, 8))
     d.close()
+
+
+def test_a_limit_that_any_wait_may_exceed(T):
+    """With a limit of a nanosecond each wait may run out or not, in any warp: a solve
+    converges or gives up, and what follows on the context is as before."""
+    from three_part_dwf_study_b200 import _capi as A
+    rng = np.random.default_rng(4)
+    d = T.DomainWall(24, 20, 6, 1.0, 0.1)
+    d.set_gauge(quenched_theta(rng, 24, 20, 3.0))
+    src = sources(rng, 9, d)
+
+    def solves():
+        return [d.propagators(src, rtol=1e-8, maxiter=3000, solver=s)[0]
+                for s in (T.SOLVER_EO_MIXED, T.SOLVER_MIXED, T.SOLVER_CG64)]
+
+    before = solves()
+    for _ in range(5):
+        A.check(A.lib().dwf_set_wait_limit(d.handle, 1), d.handle)
+        try:
+            solves()
+        except RuntimeError as e:
+            assert "ran out" in str(e)
+        A.check(A.lib().dwf_set_wait_limit(d.handle, 5_000_000_000), d.handle)
+        assert all(np.array_equal(a, b) for a, b in zip(solves(), before))
+    d.close()

@@ -2,8 +2,8 @@
 // right-hand side, for lattices whose search direction and operator temporary
 // fit a cluster's shared memory: Wilson lattices and the smaller domain-wall ones.
 //
-// There the grid-wide kernels are bound by the latency of their grid barriers (4.5 us
-// an iteration for one right-hand side, 18 for a batch of 16 at 48x40), however
+// There the grid-wide kernels are bound by the latency of their grid barriers (4.9 us
+// an iteration for one right-hand side at 32x32, 16 for a batch of 16 at 48x40), however
 // little there is to compute. Here CTA c of a cluster holds time rows [c R, (c+1) R)
 // for every slice; NL threads own a 4-D site, LT = ceil(Ls / NL) slices each, with
 // r and the iterate (FP64) or the correction e (mixed) in registers; shared memory
@@ -549,7 +549,7 @@ const void* kernel_of(bool mixed, bool fifth, int LT, int NL)
 }
 
 // Estimated time (us) of an iteration over the whole batch on the grid-wide kernels
-// (measured: one right-hand side 64x64x16 6.7 mixed, 8.7 FP64, 24x20x10 5.7; 28 at
+// (measured: one right-hand side 64x64x16 6.6 mixed, 8.6 FP64, 24x20x10 5.9; 28 at
 // 64x64x16 89 mixed, 143 FP64, 16 at 48x40 16).
 double grid_time(const Lat& L, bool mixed, int nrhs)
 {
@@ -581,8 +581,8 @@ cudaError_t load_cg_cluster64()
 // twice) and 0.055 / 0.04 us per warp, so small LT and few warps win, and the batch
 // takes the rounds its right-hand sides need of the resident clusters. Measured (us
 // an iteration, FP64): Wilson 32x32 2.6 at 2 to 7 CTAs' rows each, 3.1 with two CTAs;
-// 12x10x6 3.3 / 3.9 / 4.7 at LT 1 / 2 / 3; 24x20x10 4.7 at LT 2, 5.2 at 3; 48x40 with 16
-// right-hand sides 2.8 (grid-wide 18); 40x40x8 5.2 (grid-wide 5.6).
+// 12x10x6 3.3 / 3.9 / 4.7 at LT 1 / 2 / 3; 24x20x10 4.6 at LT 2, 5.2 at 3; 48x40 with 16
+// right-hand sides 2.8 (grid-wide 16); 40x40x8 5.0 (grid-wide 6.2).
 cudaError_t launch_cg_cluster(SolveDesc& d, bool mixed, int device, int nsm, cudaStream_t stream,
                               cudaEvent_t before, bool* taken)
 {

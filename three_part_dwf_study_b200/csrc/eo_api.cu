@@ -58,7 +58,6 @@ int eo_cluster_wave(dwf_ctx* c, int nrhs)
         return 0;
     EoDesc e{};
     e.d.nrhs = std::min(nrhs, 2048);
-    e.d.delta = 0.1;
     bool ok = false;
     int wave = 0;
     if (launch_eo_cluster(c, e, &ok, true, &wave) != DWF_OK || !ok)

@@ -7,12 +7,11 @@
 // FP32 fields streaming through L2. Here a cluster of CS CTAs owns one
 // right-hand side at a time; CTA c holds time rows [c R, (c+1) R) (R = ceil(Nt /
 // CS), the last CTA may hold fewer) of every field for every fifth-dimension
-// slice, and the phases are separated by cluster barriers only. Right-hand sides
-// are independent, so clusters never wait for one another; each takes the
-// right-hand sides cluster_id, cluster_id + nclusters, ...
+// slice. Right-hand sides are independent, so clusters never wait for one
+// another; each takes the right-hand sides cluster_id, cluster_id + nclusters, ...
 //
 // Per iteration (FP32; the same algebra as cg_eo_mixed_kernel), each phase ended
-// by a cluster barrier:
+// by a block barrier and begun by a wait for the neighbouring CTAs' rows:
 //   P1 (even sites)  y = M5^-1 H_eo p
 //   P2 (odd sites)   t = M5 p - H_oe y, |t|^2
 //   P3 (even sites)  y = M5^dag^-1 H^dag_eo t
@@ -44,8 +43,10 @@
 // kept in registers between the phases (EREG: a quarter of the hops' loads). ncu (256
 // threads, 60 iterations): 3.3 k instructions per warp and iteration, issue 35 % of its
 // peak and shared-memory wavefronts 47 % before that last step, stalls split
-// between shared-memory latency and the exchanges' waits.
-// 64x96x16 with 56, which the grid-wide kernel had to take: 113 ms, now 43.
+// between shared-memory latency and the exchanges' waits. (These with the stop at
+// twice the tolerance; at the tolerance itself it is 456 iterations and one reliable
+// update more.) 64x96x16 with 56, which the grid-wide kernel had to take, 113 ms there
+// and 45.5 here at equal stops.
 //
 // M5^-1 (per spin an Ls x Ls bidiagonal matrix with the m_f corner, closed form
 // in eo.cuh): the two fifth-dimension recurrences run over the thread's slices in
@@ -954,7 +955,11 @@ int launch_eo_cluster(dwf_ctx* c, EoDesc& e, bool* launched, bool dry, int* wave
     // Fewer reliable updates than the grid kernel's delta of 0.1 asks for: one costs
     // about four iterations here. 64x64x16, 28 right-hand sides to 1e-12: 0.1 -> 12
     // updates, 16.2 ms; 0.03 -> 8, 15.5; 0.01 -> 6, 15.2; 24x20x8 needs 184, 188, 190
-    // iterations there, and 213 at 0.003.
+    // iterations there, and 213 at 0.003. The solutions are no further off for it:
+    // on eight sets from 46x18x13 to 62x94x16, mf 0.02 to 0.1, the mean errors at 1e-8,
+    // 1e-10 and 1e-12 agree to 2 % with those of 0.1, at 32x32x24 to 11 %; on smaller
+    // lattices, where a solve ends a few iterations apart, either is the better one (by
+    // 1.4 at 24x20x8, 2.9 at most at 16x16x4).
     cd.delta = 0.02;
     cudaLaunchConfig_t cfg;
     cudaLaunchAttribute attr;

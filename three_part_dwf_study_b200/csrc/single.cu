@@ -5,16 +5,16 @@
 // them an iteration needs. The batch kernels (solver.cu) pay, at each of their
 // two barriers, a counter increment, a poll of the counter, a reload and sum of
 // every chunk's partials by one warp and two list compactions; one iteration
-// took 18 us at 64x64x16 although its arithmetic and L2 traffic need under 2.
+// took 15 us at 64x64x16 although its arithmetic and L2 traffic need under 2.
 // Here the barrier and the sum are one step (all_sum): every block publishes
 // its partial sum in a slot of its own, tagged with the step's number, and
 // every block reads all slots until their tags match. The scalars of the
 // recurrence (alpha, beta, the stopping test) then live in registers, computed
-// by every thread from the same bits. Measured on 64x64x16 (1e-12, warm-started
-// D D^dag solves of a leapfrog trajectory, mixed): 15 us an iteration before, 7.9
-// with this kernel (FP64 15.9 and 10.4); at 128x128x24, mixed, 25.5 and 21.5.
-// Steps to it, same lattice: fence after relaxed polls 12.9 us, one warp polling
-// five slots a lane one after another 9.3, slots a 128-byte line apart 8.7.
+// by every thread from the same bits. Measured (us an iteration, mixed / FP64):
+// 64x64x16 15 / 15.9 on the batch kernels' two-barrier form, 6.6 / 8.6 here; 128x128x24
+// 25.5 / - and 20.6 / 32.9. Steps to it at 64x64x16, mixed: fence after relaxed polls
+// 12.9, one warp polling five slots a lane one after another 9.3, slots a 128-byte line
+// apart 8.7, one slot per lane 7.9, the timer out of the first polls 6.7.
 //
 // Sites are dealt to threads once per solve: with at most 512 sites per SM each
 // thread owns one site (ONE), whose neighbours and links it looks up once;

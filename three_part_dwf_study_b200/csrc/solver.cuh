@@ -39,7 +39,8 @@ struct SolveDesc
     int has_guess;
     const int* active_in;  // device [nrhs] or null: right-hand sides with 0 are left untouched
     int eigen_rule;   // stop at |r|^2 < tol^2 |b|^2 and count as Eigen's ConjugateGradient
-    double delta;     // reliable-update trigger: |r32| < delta * |r| at the last update
+    double delta;     // reliable-update trigger: |r32| < delta * |r| at the last update (the
+                      // even-odd cluster kernel has its own)
     int stall_limit;  // consecutive non-improving reliable updates before giving up
     // reliable updates run only at iterations divisible by ru_period (and at
     // maxiter), so that the right-hand sides of a batch that want one share the
