@@ -127,9 +127,9 @@ __device__ __forceinline__ void sync_global()
 // every warp's sum in shared memory; after a block barrier send() (by one warp)
 // adds them and sends the CTA's sum to every CTA's table; get() waits for the
 // table and adds it up in a fixed order, the same bits in every warp of every
-// CTA (unless the wait ran out: bad). One lane per warp polls: all threads polling, and a message per warp
-// instead of per CTA, made the mbarrier the bottleneck (2.5 us a sum at 16 CTAs of
-// 16 warps against 0.5). Thread 0 arms the slot's barrier in get(). A slot
+// CTA (unless the wait ran out: bad). One lane per warp polls: all threads polling,
+// and a message per warp instead of per CTA, made the mbarrier the bottleneck (2.5 us
+// a sum at 16 CTAs of 16 warps against 0.5). Thread 0 arms the slot's barrier in get(). A slot
 // is sent again only after every warp of every CTA has sent something that it
 // sends after its get() of that slot, and someone has waited for it.
 struct Sum
@@ -193,9 +193,10 @@ __host__ __device__ constexpr size_t sum_bytes(int nslot)
 // has read its own word there, hence the number and not a flag. True: leave.
 //
 // The word and the count of check points passed lie in shared memory (8 bytes at
-// `word`), and a solver looks at left() after its loop instead of leaving from within:
-// a register or a way out of the loop more cost the even-odd kernel spills and 1.5 %. Thread 0 counts after
-// the barrier; every solver has a block barrier before its next check point.
+// `word`), and the even-odd solver looks at left() after its loop instead of leaving
+// from within: a register or a way out of the loop more cost it spills and 1.5 %.
+// Thread 0 counts after the barrier; a solver has a block barrier before its next
+// check point.
 struct Meet
 {
     unsigned word;  // shared address
